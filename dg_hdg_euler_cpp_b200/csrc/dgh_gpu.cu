@@ -14,6 +14,7 @@
 #include "dgh_kernels_krylov.cuh"
 #include "dgh_kernels_lu.cuh"
 #include "dgh_kernels_lu2.cuh"
+#include "dgh_lu.hpp"
 #include "dgh_kernels_lockstep.cuh"
 #include "dgh_kernels_q.cuh"
 
@@ -169,9 +170,9 @@ struct dgh_ctx {
     } ilu2;
     bool ilu2d() const { return ilu() && dim == 2; }
     bool ilu() const { return cfg.preconditioner == 1; }
-    // left-looking FP64 LU: per-CTA scratch of the panels' L_qq^{-1}, U_qq^{-1}; FP64 workspace
-    // for the mixed-precision DG blocks (factored in FP64 in chunks, stored as FP32 slabs)
-    double *lu_tri = nullptr, *dg_ws = nullptr;
+    // FP64 LU: resident CTAs; FP64 workspace for the mixed-precision DG blocks of the over-integrated
+    // rule (factored in FP64 in chunks, stored as FP32 slabs)
+    double *dg_ws = nullptr;
     int lu_grid = 0, dg_ws_cells = 0;
     // per-degree autotuner: chosen factorisation variants (-1 until the first refresh) and the
     // tuning times
@@ -180,8 +181,8 @@ struct dgh_ctx {
     // grid shape of the DG block solves (solve_grid; -1 until the first DG refresh) and its tuning times
     int solve_shape = -1;
     double solve_ms[2] = {0, 0};
-    // CTAs per SM of the fused DG factorisation (1 or 2; -1 until the first fused refresh): with
-    // 1 the per-CTA FP64 slots fit L2, with 2 twice the warps hide the panel latencies
+    // CTAs per SM of the fused DG factorisation (1, or 2 for every resident one; -1 until the first
+    // fused refresh): with 1 the per-CTA FP64 slots fit L2, with more the panel latencies overlap
     int fused_ctas = -1;
     double fused_ms[2] = {0, 0};
     // GMRES
@@ -272,7 +273,7 @@ struct dgh_ctx {
     bool mixed() const { return cfg.precision != DGH_PRECISION_FP64; }
     bool half16() const { return cfg.precision == DGH_PRECISION_MIXED16; }
     float *dg_scale = nullptr;  // FP16 DG factors: per-row reciprocal scales of U
-    double *dg_slots = nullptr; // reduced-precision DG factorisation: one FP64 slot per resident LU CTA
+    double *dg_slots = nullptr; // fused DG factorisation: one FP64 slot per resident LU CTA
     int dg_slot_count = 0;
     bool d1() const { return dim == 1; }
     bool overint() const { return dim == 2 && Q > n; }
@@ -499,21 +500,6 @@ void interior_cells(const dgh_ctx *c, int &first, int &count) {
     count = c->slabbed() ? c->g.nx * c->slab.rows : c->cells;
 }
 
-// The dynamic shared-memory cap of a kernel is process-wide state that every context shares (and
-// the contexts of a batch run on several host threads): it only ever rises, under a lock, so no
-// launch sees a cap below the size it was launched with.
-void allow_dynamic_smem(const void *fn, size_t bytes) {
-    static std::mutex mu;
-    static std::map<std::pair<const void *, int>, size_t> cap;
-    int dev = 0;
-    ck(cudaGetDevice(&dev), "cudaGetDevice");
-    std::lock_guard<std::mutex> lock(mu);
-    size_t &cur = cap[{fn, dev}];
-    if (bytes <= cur) return;
-    ck(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "shared memory attribute");
-    cur = bytes;
-}
-
 // Panel width 32; U12 tile width 32 for FP64 (two CTAs per SM fit in shared memory at m = 324)
 // and 64 for FP32.
 constexpr int LU_NB = 32;
@@ -534,29 +520,21 @@ void launch_lu(dgh_ctx *c, TF *pool, size_t stride, int m, int ld, int count, in
                                                                slab_out ? 3 : lfix ? 2 : 0);
     c->launched();
 }
-// The left-looking FP64 LU (dgh_kernels_lu2.cuh): grid = resident CTAs, each with its scratch.
-template <bool AUG>
-void launch_lu_left(dgh_ctx *c, double *pool, size_t stride, int m, int ld, int count, int *perm, int bit, bool slab_out,
-                    float *out32 = nullptr, double *x_out = nullptr, double *y_out = nullptr) {
-    need(m <= 2 * LL_THREADS && m % 4 == 0, "LU block width unsupported by the left-looking kernel");
-    const size_t smem = lu_left_smem_bytes(m);
-    allow_dynamic_smem((const void *)k_lu_left<AUG>, smem);
-    const int grid = std::min(count, c->lu_grid);
-    k_lu_left<AUG><<<grid, LL_THREADS, smem, c->stream>>>(pool, stride, m, ld, count, c->lu_tri, perm, c->status, bit,
-                                                          slab_out ? 1 : 0, out32, x_out, y_out);
+// The FP64 LU on the tensor pipe (dgh_kernels_lu2.cuh) of m x m blocks, in place or to FP32 slabs.
+void launch_lu_pool(dgh_ctx *c, double *pool, int m, int count, int *perm, int bit, bool slab_out, float *out32 = nullptr) {
+    lu_pool({c->stream, c->sms, c->status, bit}, pool, m, count, perm, slab_out, out32);
+    c->launched();
+}
+// The same with t + 1 augmented columns: X | y = A^{-1} [B | r], to x and y.
+void launch_lu_augmented(dgh_ctx *c, double *aug, int m, int t, int count, int *perm, int bit, double *x, double *y) {
+    lu_augmented({c->stream, c->sms, c->status, bit}, aug, m, t, count, perm, x, y);
     c->launched();
 }
 // The DG blocks of cells [first, first + count) assembled and factored in one persistent launch
-// (k_lu_left's fused mode: each CTA assembles a cell into its own FP64 slot, factors it there and
-// writes FP32 slabs, or FP16 slabs with row scales).  Collocated volume rule only.
-template <int N> void launch_dg_fused(dgh_ctx *c, int first, int count) {
-    const size_t smem = lu_left_smem_bytes(c->m);
-    allow_dynamic_smem((const void *)k_lu_left<false, N>, smem);
-    int per_sm = 0;
-    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lu_left<false, N>, LL_THREADS, smem), "occupancy");
-    const int per = std::min(std::max(1, per_sm), c->fused_ctas > 0 ? c->fused_ctas : 2);
-    const int grid = std::min(count, std::min(c->dg_slot_count, c->sms * per));
-    need(grid <= c->lu_grid, "fused factorisation grid exceeds the LU scratch");
+// (k_lu_crout's fused mode: each CTA assembles a cell into its own FP64 slot, factors it there and
+// writes FP64 or FP32 slabs, or FP16 slabs with row scales).  Collocated volume rule only.
+void launch_dg_fused(dgh_ctx *c, int first, int count) {
+    const int grid = std::min(count, c->fused_ctas == 1 ? std::min(c->dg_slot_count, c->sms) : c->dg_slot_count);
     LLFuse fu;
     fu.vol = c->vol;
     fu.fcache = c->fcache;
@@ -566,17 +544,17 @@ template <int N> void launch_dg_fused(dgh_ctx *c, int first, int count) {
     fu.g = c->g;
     fu.inv_step = c->inv_step;
     fu.first = first;
-    const size_t mp8 = pad8(c->m);
+    const size_t mp8 = pad8(c->m), at = (size_t)first * c->m * c->m;
     float *out32 = nullptr;
     if (c->half16()) {
         fu.out16 = (__half *)c->dg_pool + (size_t)first * c->m * mp8;
         fu.scale16 = c->dg_scale + (size_t)first * c->m;
+    } else if (c->mixed()) {
+        out32 = (float *)c->dg_pool + at;
     } else {
-        out32 = (float *)c->dg_pool + (size_t)first * c->m * c->m;
+        fu.out64 = (double *)c->dg_pool + at;
     }
-    k_lu_left<false, N><<<grid, LL_THREADS, smem, c->stream>>>(c->dg_slots, (size_t)c->m * c->m, c->m, c->m, count,
-                                                                c->lu_tri, c->dg_perm + (size_t)first * c->m, c->status,
-                                                                ST_SINGULAR, 0, out32, nullptr, nullptr, fu);
+    lu_fused({c->stream, c->sms, c->status, ST_SINGULAR}, c->n, fu, grid, count, c->dg_perm + (size_t)first * c->m, out32);
     c->launched();
 }
 
@@ -793,7 +771,7 @@ void ilu2_build(dgh_ctx *c) {
     L.frows = upload_int(frows);
     L.brows = upload_int(brows);
     L.pairs = upload_int(pairs);
-    L.aug = c->alloc<double>((size_t)max_rows * m * (2 * m + 1));
+    L.aug = c->alloc<double>((size_t)max_rows * m * lu_aug_ld(m, m));
     L.inv = c->alloc<double>((size_t)max_rows * mm);
     L.ydummy = c->alloc<double>((size_t)max_rows * m);
     L.perm = c->alloc<int>((size_t)max_rows * m);
@@ -851,8 +829,7 @@ template <typename TF> void ilu2_factor(dgh_ctx *c) {
         const int *rows = L.frows + L.fptr[l];
         k_ilu_stage_inverse<TF><<<std::min(cnt, c->sms * 4), 256, 0, c->stream>>>(L.aug, diag, rows, cnt, m);
         c->launched();
-        launch_lu_left<true>(c, L.aug, (size_t)m * (2 * m + 1), m, 2 * m + 1, cnt, L.perm, ST_SINGULAR, false, nullptr,
-                             L.inv, L.ydummy);
+        launch_lu_augmented(c, L.aug, m, m, cnt, L.perm, ST_SINGULAR, L.inv, L.ydummy);
         k_ilu_store_inverse<TF><<<std::min(cnt, c->sms * 4), 256, 0, c->stream>>>(diag, L.inv, rows, cnt, m);
         c->launched();
     }
@@ -2096,7 +2073,8 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
             c->Y = c->alloc<double>((size_t)c->cells * c->m);
             c->cy = c->alloc<double>((size_t)c->cells * c->t);
             c->hrhs = c->alloc<double>(c->NT);
-            const size_t per_cell = (size_t)c->m * (c->m + c->t + 1) * (c->c32() ? sizeof(float) : sizeof(double));
+            // [A | B | r | pad] and, where X is not kept, the solved columns
+            const size_t per_cell = (size_t)c->m * (lu_aug_ld(c->m, c->t) + (c->c32() ? c->t : 0)) * sizeof(double);
             const size_t budget = (size_t)8 << 30;  // condensation workspace: at most 8 GiB
             c->aug_cells = (int)std::max<size_t>(1, std::min<size_t>(c->cells, budget / per_cell));
             c->aug_bytes = (size_t)c->aug_cells * per_cell;
@@ -2122,25 +2100,19 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
         c->g_x = c->alloc<double>(vn);
         c->gdev = c->alloc<GmresDev>(1);
         ck(cudaMemset(c->V, 0, sizeof(double) * (size_t)c->vld * (k.restart + 1)), "memset");
-        if (c->has_dg() && c->mixed()) {
+        if (c->has_dg() && !c->ilu2d() && (c->mixed() || !c->overint())) {
             if (c->overint()) {  // chunked: assembly with the over-integrated volume terms, then the LU
                 const size_t per_cell = (size_t)c->m * c->m * sizeof(double);
                 const size_t budget = (size_t)8 << 30;  // FP64 factor workspace: at most 8 GiB
                 c->dg_ws_cells = (int)std::max<size_t>(1, std::min<size_t>(c->cells, budget / per_cell));
                 c->dg_ws = c->alloc<double>((size_t)c->dg_ws_cells * c->m * c->m);
-            } else {  // one persistent fused launch: an FP64 slot per resident CTA (two per SM)
-                c->dg_slot_count = std::min(c->cells, 2 * c->sms);
+            } else {  // one persistent fused launch: an FP64 slot per resident CTA
+                c->dg_slot_count = std::min(c->cells, c->sms * lu_fused_resident(c->n));
                 c->dg_slots = c->alloc<double>((size_t)c->dg_slot_count * c->m * c->m);
             }
         }
         if (c->has_dg() || c->has_hdg()) {
-            const size_t smem = lu_left_smem_bytes(c->m);
-            allow_dynamic_smem((const void *)k_lu_left<true>, smem);
-            int per_sm = 0;
-            ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lu_left<true>, LL_THREADS, smem), "occupancy");
-            c->lu_grid = c->sms * std::max(1, per_sm);
-            const int P = (c->m + LL_NB - 1) / LL_NB;
-            c->lu_tri = c->alloc<double>((size_t)c->lu_grid * P * LL_TRI);
+            c->lu_grid = c->sms * lu_resident(c->m, c->has_hdg());
         }
         if (c->has_dg() && c->ilu2d()) ilu2_build(c);
         if (c->slabbed()) c->slab.buf = c->alloc<double>(16);
@@ -2627,9 +2599,9 @@ std::map<std::tuple<int, int, int, int>, int> g_tune_cache;  // (kind, n, precis
 void dg_factor(dgh_ctx *c, int variant, int first, int count) {
     const size_t stride = (size_t)c->m * c->m;
     const int grid = std::min(count, c->sms * 8);
-    if (c->mixed() && (c->half16() || variant == 0) && !c->overint()) {
-        // one persistent launch: assemble + FP64 left-looking LU per CTA slot, reduced output
-        DGH_DISPATCH_N(c->n, { launch_dg_fused<N>(c, first, count); });
+    if ((c->half16() || variant == 0) && !c->overint()) {
+        // one persistent launch: assembly and FP64 LU in per-CTA slots, slabs out
+        launch_dg_fused(c, first, count);
         return;
     }
     if (c->half16()) {  // FP64 left-looking in the workspace, then FP16 slabs with row scales
@@ -2646,7 +2618,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
                 }
             });
             c->launched();
-            launch_lu_left<false>(c, c->dg_ws, stride, c->m, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR, false);
+            launch_lu_pool(c, c->dg_ws, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR, false);
             const long long warps = (long long)cnt * ((c->m + 31) / 32);
             k_pack_half<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, c->stream>>>(
                 c->dg_ws, c->m, cnt, (__half *)c->dg_pool + (size_t)f * c->m * mp, c->dg_scale + (size_t)f * c->m);
@@ -2668,8 +2640,8 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
                     }
                 });
                 c->launched();
-                launch_lu_left<false>(c, c->dg_ws, stride, c->m, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR,
-                                      false, (float *)c->dg_pool + (size_t)f * stride);
+                launch_lu_pool(c, c->dg_ws, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR, false,
+                               (float *)c->dg_pool + (size_t)f * stride);
             }
         } else {  // FP32 right-looking in place
             float *pool = (float *)c->dg_pool + (size_t)first * stride;
@@ -2698,7 +2670,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
         });
         c->launched();
         if (variant == 0)
-            launch_lu_left<false>(c, pool, stride, c->m, c->m, count, c->dg_perm + (size_t)first * c->m, ST_SINGULAR, true);
+            launch_lu_pool(c, pool, c->m, count, c->dg_perm + (size_t)first * c->m, ST_SINGULAR, true);
         else
             launch_lu<double>(c, pool, stride, c->m, c->m, count, c->dg_perm + (size_t)first * c->m, ST_SINGULAR, true);
     }
@@ -2706,7 +2678,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
 // Condensation of cells [first, first + count) (count <= aug_cells): [A | B | r], LU + solve
 // with the given variant, S, X, y, C y.
 void hdg_condense_chunk(dgh_ctx *c, int variant, const double *r, int first, int count) {
-    const int ld = c->m + c->t + 1, grid = std::min(count, c->sms * 8);
+    const int ld = lu_aug_ld(c->m, c->t), grid = std::min(count, c->sms * 8);
     DGH_DISPATCH_N(c->n, {
         k_hdg_assemble<N, double><<<grid, 256, 0, c->stream>>>(c->aug, c->vol, c->fcache, c->speeds, r, c->basis, c->g,
                                                                c->inv_step, first, count, c->overint() ? 0 : 1);
@@ -2718,8 +2690,8 @@ void hdg_condense_chunk(dgh_ctx *c, int variant, const double *r, int first, int
     });
     c->launched();
     if (variant == 0) {  // X and y straight to their persistent arrays
-        launch_lu_left<true>(c, c->aug, (size_t)c->m * ld, c->m, ld, count, c->aug_perm, ST_SINGULAR_HDG, false, nullptr,
-                             c->X + (size_t)first * c->m * c->t, c->Y + (size_t)first * c->m);
+        launch_lu_augmented(c, c->aug, c->m, c->t, count, c->aug_perm, ST_SINGULAR_HDG, c->X + (size_t)first * c->m * c->t,
+                            c->Y + (size_t)first * c->m);
     } else {
         launch_lu<double>(c, c->aug, (size_t)c->m * ld, c->m, ld, count, c->aug_perm, ST_SINGULAR_HDG, false);
         constexpr size_t bs_smem = backsolve_smem_bytes();
@@ -2740,17 +2712,20 @@ void hdg_condense_chunk(dgh_ctx *c, int variant, const double *r, int first, int
     });
     c->launched();
 }
-// Cells per chunk of the condensation workspace for augmented matrices of element type T.
+// Cells per chunk of the FP32-storage condensation's workspace: augmented matrices of element type T
+// and, in the FP64 form, their solved columns X.
 template <typename T> int aug_chunk(const dgh_ctx *c) {
-    return (int)std::max<size_t>(1, std::min<size_t>(c->cells, c->aug_bytes / ((size_t)c->m * (c->m + c->t + 1) *
-                                                                                 sizeof(T))));
+    const size_t row = lu_aug_ld(c->m, c->t) + (sizeof(T) == 8 ? c->t : 0);
+    return (int)std::max<size_t>(1, std::min<size_t>(c->cells, c->aug_bytes / ((size_t)c->m * row * sizeof(T))));
 }
 // FP32-storage condensation of cells [first, first + count), variant 0: [A | B | r] assembled in
-// FP64, the left-looking LU on the FP64 tensor pipe with the fused right-hand-side solve, the
-// factors rounded into the cells' FP32 slabs, then S = -C X stored in FP32, y and C y in FP64.
+// FP64, the LU on the FP64 tensor pipe with the fused right-hand-side solve (X behind the matrices
+// in the workspace), the factors rounded into the cells' FP32 slabs, then S = -C X stored in FP32, y
+// and C y in FP64.
 void hdg_condense_chunk32_tc(dgh_ctx *c, const double *r, int first, int count) {
-    const int ld = c->m + c->t + 1, grid = std::min(count, c->sms * 8);
+    const int ld = lu_aug_ld(c->m, c->t), grid = std::min(count, c->sms * 8);
     const size_t stride = (size_t)c->m * ld;
+    double *X = c->aug + (size_t)aug_chunk<double>(c) * stride;
     DGH_DISPATCH_N(c->n, {
         k_hdg_assemble<N, double><<<grid, 256, 0, c->stream>>>(c->aug, c->vol, c->fcache, c->speeds, r, c->basis, c->g,
                                                                c->inv_step, first, count, c->overint() ? 0 : 1);
@@ -2762,14 +2737,14 @@ void hdg_condense_chunk32_tc(dgh_ctx *c, const double *r, int first, int count) 
     });
     c->launched();
     int *perm = c->lu32_perm + (size_t)first * c->m;
-    launch_lu_left<true>(c, c->aug, stride, c->m, ld, count, perm, ST_SINGULAR_HDG, false);
+    launch_lu_augmented(c, c->aug, c->m, c->t, count, perm, ST_SINGULAR_HDG, X, c->Y + (size_t)first * c->m);
     const long long warps = (long long)count * ((c->m + 31) / 32);
     k_slab_pack<double, float><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, c->stream>>>(
         c->aug, stride, c->m, ld, count, c->lu32 + (size_t)first * c->m * c->m, perm);
     c->launched();
     DGH_DISPATCH_N(c->n, {
-        k_hdg_schur<N, double, false, float><<<grid, 256, 0, c->stream>>>(c->aug, c->fcache, c->speeds, c->S32, nullptr,
-                                                                          c->Y, c->cy, c->basis, c->g, first, count);
+        k_hdg_schur<N, double, true, float><<<grid, 256, 0, c->stream>>>(nullptr, c->fcache, c->speeds, c->S32, X, c->Y,
+                                                                         c->cy, c->basis, c->g, first, count, 0, first);
     });
     c->launched();
 }
@@ -2777,7 +2752,7 @@ void hdg_condense_chunk32_tc(dgh_ctx *c, const double *r, int first, int count) 
 // fix-up kept), the factors copied to the cells' FP32 slabs for later solves, back substitution
 // for X | y, then S = -C X stored in FP32, y and C y in FP64.
 void hdg_condense_chunk32(dgh_ctx *c, const double *r, int first, int count) {
-    const int ld = c->m + c->t + 1, grid = std::min(count, c->sms * 8);
+    const int ld = lu_aug_ld(c->m, c->t), grid = std::min(count, c->sms * 8);
     const size_t stride = (size_t)c->m * ld;
     DGH_DISPATCH_N(c->n, {
         k_hdg_assemble<N, float><<<grid, 256, 0, c->stream>>>(c->aug32, c->vol, c->fcache, c->speeds, r, c->basis, c->g,
@@ -2940,7 +2915,7 @@ int dgh_block_jacobi_refresh(dgh_ctx *c, int op) {
                 c->check_status();
             }
             if (c->fused_ctas < 0) {  // the fused path's residency (kind 4): 1 or 2 CTAs per SM
-                const bool fused = c->mixed() && (c->half16() || c->dg_variant == 0) && !c->overint();
+                const bool fused = (c->half16() || c->dg_variant == 0) && !c->overint();
                 if (fused) {
                     const int sample = std::min(c->cells, std::max(c->lu_grid, 1) * 4);
                     const int v = tuned_variant_all(c, 4, [&](int k) {
@@ -3225,7 +3200,7 @@ int dgh_block_jacobi_create(int m, int count, int precision, int variant, int de
     bj->c = new dgh_ctx;
     dgh_ctx *c = bj->c;
     const int rc = guard(c, [&] {
-        need(m >= 1 && count >= 1 && m <= 2 * LL_THREADS, "Invalid block size or count");
+        need(m >= 1 && count >= 1 && m <= LU_MAX_WIDTH, "Invalid block size or count");
         need(precision == DGH_PRECISION_FP64 || precision == DGH_PRECISION_MIXED, "Invalid precision");
         need(variant >= 0 && variant <= 3, "Invalid factorisation variant");
         need(variant != 0 || m % 4 == 0, "LU block width unsupported by the left-looking kernel");
@@ -3252,14 +3227,6 @@ int dgh_block_jacobi_create(int m, int count, int precision, int variant, int de
         const size_t tsz = precision == DGH_PRECISION_MIXED ? sizeof(float) : sizeof(double);
         bj->pool = c->alloc<char>((size_t)count * m * m * tsz);
         bj->perm = c->alloc<int>((size_t)count * m);
-        if (variant == 0) {
-            const size_t smem = lu_left_smem_bytes(m);
-            allow_dynamic_smem((const void *)k_lu_left<false>, smem);
-            int per_sm = 0;
-            ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lu_left<false>, LL_THREADS, smem), "occupancy");
-            c->lu_grid = c->sms * std::max(1, per_sm);
-            c->lu_tri = c->alloc<double>((size_t)c->lu_grid * ((m + LL_NB - 1) / LL_NB) * LL_TRI);
-        }
         if (precision == DGH_PRECISION_MIXED && (variant == 0 || variant == 3))
             bj->ws = c->alloc<double>((size_t)count * m * m);
         c->sync();
@@ -3295,7 +3262,7 @@ int dgh_block_jacobi_factor(dgh_block_jacobi *bj, const double *blocks) {
         if (bj->precision == DGH_PRECISION_FP64) {
             double *pool = (double *)bj->pool;
             ck(cudaMemcpyAsync(pool, blocks, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy blocks");
-            if (bj->variant == 0) launch_lu_left<false>(c, pool, stride, m, m, count, bj->perm, ST_SINGULAR, true);
+            if (bj->variant == 0) launch_lu_pool(c, pool, m, count, bj->perm, ST_SINGULAR, true);
             else if (bj->variant == 1) launch_lu<double>(c, pool, stride, m, m, count, bj->perm, ST_SINGULAR, true);
             else launch_lu_narrow<double>(c, pool, m, count, bj->perm, ST_SINGULAR);
         } else {
@@ -3303,7 +3270,7 @@ int dgh_block_jacobi_factor(dgh_block_jacobi *bj, const double *blocks) {
             if (bj->variant == 0 || bj->variant == 3) {
                 ck(cudaMemcpyAsync(bj->ws, blocks, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy blocks");
                 if (bj->variant == 0) {
-                    launch_lu_left<false>(c, bj->ws, stride, m, m, count, bj->perm, ST_SINGULAR, false, pool);
+                    launch_lu_pool(c, bj->ws, m, count, bj->perm, ST_SINGULAR, false, pool);
                 } else {
                     const size_t smem = inv_narrow_smem_bytes(m);
                     allow_dynamic_smem((const void *)k_inv_narrow, smem);

@@ -6,6 +6,7 @@
 // factorisation are plain GEMMs (cuBLAS), and the diagonal inverses come from k_lu_left.
 #pragma once
 #include "dgh_kernels_dg.cuh"
+#include "dgh_lu.hpp"
 
 namespace dgh {
 
@@ -71,11 +72,11 @@ __global__ void k_copy_blocks(TF *const *__restrict__ dst, const TF *const *__re
 }
 
 // [A_ii | I | 0] in FP64 (row length 2m + 1) from the stored diagonal blocks of the listed rows,
-// for k_lu_left's augmented solve: X = A_ii^{-1}.
+// for the augmented LU's solve: X = A_ii^{-1}.
 template <typename TF>
 __global__ void k_ilu_stage_inverse(double *__restrict__ aug, const TF *__restrict__ diag, const int *__restrict__ rows,
                                     int count, int m) {
-    const int ld = 2 * m + 1;
+    const int ld = lu_aug_ld(m, m);
     for (int k = blockIdx.x; k < count; k += gridDim.x) {
         const TF *a = diag + (size_t)rows[k] * m * m;
         double *o = aug + (size_t)k * m * ld;
