@@ -9,50 +9,46 @@
 
 namespace dgh {
 
-// Augmented rows [m][ld], ld = lu_aug_ld(m, t), t = 16 N, for cells first..first+count-1: zeros (16-byte
-// stores), then the entries that are not zero (the cross of nodes sharing a line with the row's node, four
-// trace columns and the residual), a fifth of the row; evaluating every entry took 4.3 ms per 6,900 cells
-// at k = 8, against the 1.3 ms the stores take.
+// Augmented rows [m][ld], ld = lu_aug_ld(m, t), t = 16 N, for cells first..first+count-1: the cell
+// block, the four trace columns each row couples to, the residual.
 template <int N, typename TF>
 __global__ void __launch_bounds__(256)
 k_hdg_assemble(TF *__restrict__ aug, const double *__restrict__ vol, const double *__restrict__ fcache,
                const double *__restrict__ speeds, const double *__restrict__ rvol, Basis1D b, Grid g,
                double inv_step, int first, int count, int volterm = 1) {
-    constexpr int P = N * N, M = NVAR * P, FW = NVAR * N, T = NFACES * FW, LD = lu_aug_ld(M, T), X = 2 * N - 1;
-    constexpr int ENTRIES = NVAR * X + NFACES + 1;  // per row
+    constexpr int P = N * N, M = NVAR * P, FW = NVAR * N, T = NFACES * FW, LD = lu_aug_ld(M, T), R = rows_at_once(LD, M);
     __shared__ double jx[P * 16], jy[P * 16], fj[NFACES * N * 16], stab[NFACES * N];
+    __shared__ __align__(16) double buf[R * LD];
     __shared__ Basis1D sb;
     stage_basis<N>(b, sb);
     for (int blk = blockIdx.x; blk < count; blk += gridDim.x) {
         const int cell = first + blk;
         __syncthreads();
-        TF *A = aug + (size_t)blk * M * LD;
-        for (int idx = threadIdx.x; idx < (int)(M * LD * sizeof(TF) / 16); idx += blockDim.x)
-            reinterpret_cast<float4 *>(A)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
         cell_tables<N, true>(cell, vol, fcache, speeds, sb, g, jx, jy, fj);
         for (int k = threadIdx.x; k < NFACES * N; k += blockDim.x) {
             const int side = k / N, q = k % N, face = face_of(g, cell, side);
             const double tau = speeds[2 * (face * N + q) + (side % 2 ? 0 : 1)];
             stab[k] = face_weight(g, sb, face, q) * tau;
         }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < M * ENTRIES; idx += blockDim.x) {
-            const int r = idx / ENTRIES, e = idx % ENTRIES, v = r / P, node = r % P, ix = node % N, iy = node / N;
-            int col;
-            double val;
-            if (e < NVAR * X) {
-                const int w = e / X, k = e % X, q = k - N;
-                col = w * P + (k < N ? k + N * iy : ix + N * (q + (q >= iy)));
-                val = cell_block_entry<N>(r, col, jx, jy, fj, sb, g, inv_step, volterm != 0);
-            } else if (e < NVAR * X + NFACES) {
-                const int side = e - NVAR * X, q = side < 2 ? iy : ix;
-                col = M + side * FW + v * N + q;
-                val = -stab[side * N + q] * (side % 2 ? sb.eR : sb.eL)[side < 2 ? ix : iy];
-            } else {
-                col = M + T;
-                val = rvol[(size_t)cell * M + r];
+        for (int r0 = 0; r0 < M; r0 += R) {
+            const int rows = min(R, M - r0);
+            for (int i = threadIdx.x; i < rows * LD; i += blockDim.x) buf[i] = 0.;
+            __syncthreads();
+            cell_rows_fill<N>(buf, LD, r0, rows, jx, jy, fj, sb, g, inv_step, volterm != 0, blockDim.x);
+            for (int idx = threadIdx.x; idx < rows * (NFACES + 1); idx += blockDim.x) {
+                const int side = idx % (NFACES + 1), i0 = idx / (NFACES + 1), r = r0 + i0;
+                const int v = r / P, node = r % P, ix = node % N, iy = node / N;
+                double *row = buf + (size_t)i0 * LD + M;
+                if (side < NFACES) {
+                    const int q = side < 2 ? iy : ix;
+                    row[side * FW + v * N + q] = -stab[side * N + q] * (side % 2 ? sb.eR : sb.eL)[side < 2 ? ix : iy];
+                } else {
+                    row[T] = rvol[(size_t)cell * M + r];
+                }
             }
-            A[(size_t)r * LD + col] = (TF)val;
+            __syncthreads();
+            rows_out(aug + (size_t)blk * M * LD + (size_t)r0 * LD, buf, rows * LD, blockDim.x);
+            __syncthreads();
         }
     }
 }

@@ -757,22 +757,6 @@ __device__ __forceinline__ void ll_stage_row(double *dst, const double *src, int
     }
 }
 
-// The cell block's entries (cell_block_entry) into A (row length ld): zeros, then the cross of nodes
-// that share a line with the row's node, which is all that is not zero (4 (2 N - 1) of 4 N^2 a row).
-template <int N>
-__device__ __forceinline__ void cr_assemble(double *A, int ld, const double *jx, const double *jy, const double *fj,
-                                            const Basis1D &b, const Grid &g, double inv_step, int threads) {
-    constexpr int P = N * N, M = NVAR * P, X = 2 * N - 1;
-    for (int idx = threadIdx.x; idx < M * (M / 2); idx += threads)
-        *reinterpret_cast<double2 *>(A + (size_t)(idx / (M / 2)) * ld + idx % (M / 2) * 2) = make_double2(0., 0.);
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < M * NVAR * X; idx += threads) {
-        const int r = idx / (NVAR * X), w = idx / X % NVAR, k = idx % X, node = r % P, ix = node % N, iy = node / N;
-        const int q = k - N, col = w * P + (k < N ? k + N * iy : ix + N * (q + (q >= iy)));
-        A[(size_t)r * ld + col] = cell_block_entry<N>(r, col, jx, jy, fj, b, g, inv_step, true);
-    }
-}
-
 // Batched LU.  AUG = false: pool holds m x m blocks (ld = m); on exit row i of each block is position i
 // of the factors (unit L below, U on and above the diagonal), perm_out[i] = its original row, and with
 // slab_out the block is rewritten in the slab layout of k_lu_solve.  With out32 != nullptr the factors
@@ -793,13 +777,22 @@ k_lu_crout(double *pool, size_t stride, int m, int ld, int t, int count, int *__
     for (int blk = blockIdx.x; blk < count; blk += gridDim.x) {
         double *A = pool + (size_t)blk * stride;
         if constexpr (FN > 0) {
-            // assemble the cell's block into this CTA's slot (tables in the panel area)
-            constexpr int FP = FN * FN, FM = NVAR * FP;
+            // assemble the cell's block into this CTA's slot (tables and rows in the panel area)
+            constexpr int FP = FN * FN, FM = NVAR * FP, TABLES = 2 * FP * 16 + NFACES * FN * 16;
+            constexpr int R = (cr_area(FM) - TABLES) / FM < FM ? (cr_area(FM) - TABLES) / FM : FM;
             A = fu.slots + (size_t)blockIdx.x * FM * FM;
-            double *jx = s.acc, *jy = jx + FP * 16, *fj = jy + FP * 16;
+            double *jx = s.acc, *jy = jx + FP * 16, *fj = jy + FP * 16, *buf = fj + NFACES * FN * 16;
             __syncthreads();
             cell_tables<FN, false>(fu.first + blk, fu.vol, fu.fcache, fu.speeds, fsb, fu.g, jx, jy, fj);
-            cr_assemble<FN>(A, FM, jx, jy, fj, fsb, fu.g, fu.inv_step, T);
+            for (int r0 = 0; r0 < FM; r0 += R) {
+                const int rows = min(R, FM - r0);
+                for (int i = tid; i < rows * FM / 2; i += T) reinterpret_cast<double2 *>(buf)[i] = make_double2(0., 0.);
+                __syncthreads();
+                cell_rows_fill<FN>(buf, FM, r0, rows, jx, jy, fj, fsb, fu.g, fu.inv_step, true, T);
+                __syncthreads();
+                rows_out(A + (size_t)r0 * FM, buf, rows * FM, T);
+                __syncthreads();
+            }
         }
         if (tid == 0) *s.bad = 0;
         __syncthreads();
