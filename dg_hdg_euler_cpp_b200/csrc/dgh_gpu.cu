@@ -974,7 +974,8 @@ void hdg_apply(dgh_ctx *c, const double *lam, double *out) {
     }
     slab_trace_halo(c, lam);
     DGH_DISPATCH_N(c->n, {
-        if (c->c32()) k_hdg_apply32<N><<<c->faces, 256, 0, c->stream>>>(c->S32, c->speeds, lam, out, c->basis, c->g);
+        if (c->c32())
+            k_hdg_apply32<N><<<c->faces, schur32_threads<N>(), 0, c->stream>>>(c->S32, c->speeds, lam, out, c->basis, c->g);
         else k_hdg_apply<N><<<c->faces, 256, 0, c->stream>>>(c->S, c->speeds, lam, out, c->basis, c->g);
     });
     c->launched();
@@ -1280,7 +1281,7 @@ void ls_jv_all(dgh_lockstep *L, int src, int dst, int gate) {
     for (const auto &r : L->degrees) {
         if (L->op == DGH_OP_HDG) {
             DGH_DISPATCH_N(r.key, {
-                k_ls_hdg_apply<N><<<r.blocks, 256, 0, L->stream>>>(L->table, r.first, r.count, src, dst, gate);
+                k_ls_hdg_apply<N><<<r.blocks, ls_schur_threads<N>(), 0, L->stream>>>(L->table, r.first, r.count, src, dst, gate);
             });
             L->launched();
             continue;

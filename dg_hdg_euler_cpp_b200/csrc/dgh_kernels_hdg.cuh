@@ -186,45 +186,69 @@ __device__ __forceinline__ double widen_scaled(float f) {
 }
 // (The Schur-apply bodies take their face explicitly, so the batched kernels of a lockstep
 // batch run the same arithmetic per member; every rounding is explicit: fma() and rfma.)
+// Threads of an FP32 Schur-apply CTA: rows of T / 4 float4 column groups, as many rows side by side as fit
+// 288 threads (8 at k = 8), so that every thread has a column group and keeps the group's trace values of
+// both cells in registers for all its rows.  (A warp per row left 28 of 32 lanes idle in the second of
+// its two passes over a row's 36 groups at k = 8, and read every trace value from shared memory once per
+// row: 1.35 ms at 256 x 256 against 0.85 ms for the blocks' bytes at the copy rate.)
+template <int N> __host__ __device__ constexpr int schur32_rows() { return 288 / (4 * N) < 4 * N ? 288 / (4 * N) : 4 * N; }
+template <int N> __host__ __device__ constexpr int schur32_threads() { return (schur32_rows<N>() * 4 * N + 31) / 32 * 32; }
 template <int N>
 __device__ __forceinline__ void hdg_apply32_body(int face, const float *__restrict__ S, const double *__restrict__ speeds,
                                                  const double *__restrict__ lam, double *__restrict__ out,
                                                  const Basis1D &b, const Grid &g) {
-    constexpr int FW = NVAR * N, T = NFACES * FW, T4 = T / 4, PASSES = (T4 + 31) / 32;
+    constexpr int FW = NVAR * N, T = NFACES * FW, T4 = T / 4, R = schur32_rows<N>(), PASSES = (FW + R - 1) / R;
     constexpr double kScale = 0x1p896;  // undoes the 2^-896 of widen_scaled
-    __shared__ __align__(16) double loc[2][T];
+    __shared__ double part[FW][T4 + 1];
     const int axis = face >= g.cells, first = face - axis * g.cells, next = neighbor(g, first, 2 * axis + 1);
-    for (int k = threadIdx.x; k < 2 * T; k += blockDim.x) {
-        const int which = k / T, s = (k % T) / FW, j = k % FW;
-        const int cell = which ? next : first;
-        loc[which][k % T] = kScale * lam[(size_t)face_of(g, cell, s) * FW + j];
+    const int tid = threadIdx.x, j = tid % T4, r0 = tid / T4;
+    // the rows of a face's side in S_K are contiguous: T floats each, a multiple of four
+    const float4 *s1 = reinterpret_cast<const float4 *>(S + (size_t)first * T * T + (size_t)(2 * axis + 1) * FW * T) + j;
+    const float4 *s2 = reinterpret_cast<const float4 *>(S + (size_t)next * T * T + (size_t)(2 * axis) * FW * T) + j;
+    float4 a[PASSES], c[PASSES];
+#pragma unroll
+    for (int p = 0; p < PASSES; ++p) {
+        const int row = r0 + p * R;
+        if (tid < R * T4 && row < FW) {
+            a[p] = __ldg(s1 + (size_t)row * T4);
+            c[p] = __ldg(s2 + (size_t)row * T4);
+        }
+    }
+    double x[4], y[4];
+    {
+        const int s = 4 * j / FW, k = 4 * j % FW;  // FW is a multiple of four: a group stays on one side
+        const double *l1 = lam + (size_t)face_of(g, first, s) * FW + k, *l2 = lam + (size_t)face_of(g, next, s) * FW + k;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            x[e] = kScale * l1[e];
+            y[e] = kScale * l2[e];
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < PASSES; ++p) {
+        const int row = r0 + p * R;
+        if (tid < R * T4 && row < FW) {
+            double acc = rmul(widen_scaled(a[p].x), x[0]);
+            acc = fma(widen_scaled(a[p].y), x[1], acc);
+            acc = fma(widen_scaled(a[p].z), x[2], acc);
+            acc = fma(widen_scaled(a[p].w), x[3], acc);
+            acc = fma(widen_scaled(c[p].x), y[0], acc);
+            acc = fma(widen_scaled(c[p].y), y[1], acc);
+            acc = fma(widen_scaled(c[p].z), y[2], acc);
+            acc = fma(widen_scaled(c[p].w), y[3], acc);
+            part[row][j] = acc;
+        }
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int row = warp; row < FW; row += 8) {
-        // rows of S_K are T = 16N floats (a multiple of four), so every row starts 16-byte aligned
-        const float4 *s1 = reinterpret_cast<const float4 *>(S + (size_t)first * T * T + (size_t)((2 * axis + 1) * FW + row) * T);
-        const float4 *s2 = reinterpret_cast<const float4 *>(S + (size_t)next * T * T + (size_t)((2 * axis) * FW + row) * T);
+    // row sums: 8 lanes a row, in a fixed order
+    for (int idx = tid; idx < ((FW * 8 + 31) / 32) * 32; idx += blockDim.x) {
+        const int row = idx / 8, l = idx % 8;
         double acc = 0;
+        if (row < FW)
+            for (int k = l; k < T4; k += 8) acc = radd(acc, part[row][k]);
 #pragma unroll
-        for (int t = 0; t < PASSES; ++t) {
-            const int j = lane + 32 * t;
-            if (j < T4) {
-                const float4 a = s1[j], c = s2[j];
-                const double *x = loc[0] + 4 * j, *y = loc[1] + 4 * j;
-                acc = fma(widen_scaled(a.x), x[0], acc);
-                acc = fma(widen_scaled(a.y), x[1], acc);
-                acc = fma(widen_scaled(a.z), x[2], acc);
-                acc = fma(widen_scaled(a.w), x[3], acc);
-                acc = fma(widen_scaled(c.x), y[0], acc);
-                acc = fma(widen_scaled(c.y), y[1], acc);
-                acc = fma(widen_scaled(c.z), y[2], acc);
-                acc = fma(widen_scaled(c.w), y[3], acc);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (lane == 0) {
+        for (int o = 4; o > 0; o >>= 1) acc = radd(acc, __shfl_down_sync(0xffffffffu, acc, o, 8));
+        if (row < FW && l == 0) {
             const int q = row % N;
             const double d = -face_weight(g, b, face, q) * (speeds[2 * (face * N + q)] + speeds[2 * (face * N + q) + 1]);
             out[(size_t)face * FW + row] = rfma(d, lam[(size_t)face * FW + row], acc);
@@ -232,7 +256,7 @@ __device__ __forceinline__ void hdg_apply32_body(int face, const float *__restri
     }
 }
 template <int N>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(schur32_threads<N>())
 k_hdg_apply32(const float *__restrict__ S, const double *__restrict__ speeds, const double *__restrict__ lam,
               double *__restrict__ out, Basis1D b, Grid g) {
     hdg_apply32_body<N>(blockIdx.x, S, speeds, lam, out, b, g);
@@ -252,7 +276,7 @@ __device__ __forceinline__ void hdg_apply_body(int face, const double *__restric
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double2 *l0 = reinterpret_cast<const double2 *>(loc[0]), *l1 = reinterpret_cast<const double2 *>(loc[1]);
-    for (int row = warp; row < FW; row += 8) {
+    for (int row = warp; row < FW; row += blockDim.x >> 5) {
         // rows of S_K are T = 16N doubles (an even count), so every row starts 16-byte aligned
         const double2 *s1 = reinterpret_cast<const double2 *>(S + (size_t)first * T * T + (size_t)((2 * axis + 1) * FW + row) * T);
         const double2 *s2 = reinterpret_cast<const double2 *>(S + (size_t)next * T * T + (size_t)((2 * axis) * FW + row) * T);

@@ -195,8 +195,9 @@ k_ls_inv_apply(const LsMember *t, int first, int count, int src, int dst, int j,
 }
 
 // ---- condensed Schur apply of HDG members [first, first + count), all of degree N - 1 ----------
+template <int N> __host__ __device__ constexpr int ls_schur_threads() { return schur32_threads<N>() > 256 ? schur32_threads<N>() : 256; }
 template <int N>
-__global__ void __launch_bounds__(256) k_ls_hdg_apply(const LsMember *t, int first, int count, int src, int dst,
+__global__ void __launch_bounds__(ls_schur_threads<N>()) k_ls_hdg_apply(const LsMember *t, int first, int count, int src, int dst,
                                                       int gate) {
     const LsMember &a = t[ls_find(t, first, count, blockIdx.x, LS_TEAM)];
     if (!ls_on(a, gate)) return;
