@@ -17,6 +17,7 @@
 #include "dgh_lu.hpp"
 #include "dgh_kernels_lockstep.cuh"
 #include "dgh_kernels_q.cuh"
+#include "dgh_kernels_solve.cuh"
 
 #include <cublas_v2.h>
 
@@ -502,6 +503,14 @@ void interior_cells(const dgh_ctx *c, int &first, int &count) {
 
 // Panel width 32; U12 tile width 32 for FP64 (two CTAs per SM fit in shared memory at m = 324)
 // and 64 for FP32.
+// The FP64 slabs' diagonal squares inverted in place: the last step of every factorisation that leaves FP64
+// slabs.
+void launch_slab_invert(dgh_ctx *c, double *pool, int m, int count) {
+    const long long squares = (long long)count * ((m + 31) / 32);
+    k_slab_invert<<<(unsigned)((squares + SQUARE_WARPS - 1) / SQUARE_WARPS), 32 * SQUARE_WARPS, 0, c->stream>>>(
+        pool, (size_t)m * m, m, count);
+    c->launched();
+}
 constexpr int LU_NB = 32;
 template <typename TF> constexpr int lu_tc() { return sizeof(TF) == 8 ? 32 : 64; }
 template <typename TF> void setup_lu_attrs(size_t smem) {
@@ -519,11 +528,14 @@ void launch_lu(dgh_ctx *c, TF *pool, size_t stride, int m, int ld, int count, in
     k_lu<TF, LU_NB, TC><<<grid, LU_THREADS, smem, c->stream>>>(pool, stride, m, ld, count, perm, c->status, bit,
                                                                slab_out ? 3 : lfix ? 2 : 0);
     c->launched();
+    if constexpr (sizeof(TF) == 8)
+        if (slab_out) launch_slab_invert(c, pool, m, count);
 }
 // The FP64 LU on the tensor pipe (dgh_kernels_lu2.cuh) of m x m blocks, in place or to FP32 slabs.
 void launch_lu_pool(dgh_ctx *c, double *pool, int m, int count, int *perm, int bit, bool slab_out, float *out32 = nullptr) {
     lu_pool({c->stream, c->sms, c->status, bit}, pool, m, count, perm, slab_out, out32);
     c->launched();
+    if (slab_out && !out32) launch_slab_invert(c, pool, m, count);
 }
 // The same with t + 1 augmented columns: X | y = A^{-1} [B | r], to x and y.
 void launch_lu_augmented(dgh_ctx *c, double *aug, int m, int t, int count, int *perm, int bit, double *x, double *y) {
@@ -556,6 +568,7 @@ void launch_dg_fused(dgh_ctx *c, int first, int count) {
     }
     lu_fused({c->stream, c->sms, c->status, ST_SINGULAR}, c->n, fu, grid, count, c->dg_perm + (size_t)first * c->m, out32);
     c->launched();
+    if (fu.out64) launch_slab_invert(c, fu.out64, c->m, count);
 }
 
 // Narrow blocks (m <= 64): one warp per block in shared memory.
@@ -570,6 +583,7 @@ void launch_lu_narrow(dgh_ctx *c, TF *pool, int m, int count, int *perm, int bit
     const int grid = std::min((count + wpc - 1) / wpc, c->sms * std::max(1, resident));
     k_lu_narrow<TF><<<grid, NARROW_THREADS, smem, c->stream>>>(pool, m, count, perm, c->status, bit);
     c->launched();
+    if constexpr (sizeof(TF) == 8) launch_slab_invert(c, pool, m, count);
 }
 // Grid of a one-warp-per-block solve over `count` blocks with `wpc` warps per CTA and `resident`
 // CTAs per SM.  Shape 0 fills every resident CTA slot, so the last round of blocks runs on the
@@ -584,49 +598,27 @@ int solve_grid(const dgh_ctx *c, long long count, int wpc, int resident, int sha
     const long long rounds = (count + full * wpc - 1) / (full * wpc);
     return (int)((count + wpc * rounds - 1) / (wpc * rounds));
 }
-// One warp per block; enough warps for every SM to keep its warp slots (and their loads) busy.
-// FP32 blocks narrower than two slabs (the HDG face blocks) use the register-held diagonal rows.
-template <typename TF, bool DIAG>
-void launch_solve_as(dgh_ctx *c, const TF *pool, const int *perm, size_t stride, int m, int count, const double *x,
-                     double *z, int shape) {
-    constexpr int wpc = SOLVE_THREADS / 32;
-    const size_t smem = sizeof(TF) * (size_t)m * wpc;
-    int resident = 0;
-    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_lu_solve<TF, DIAG>, SOLVE_THREADS, smem), "occupancy");
-    const int grid = solve_grid(c, count, wpc, resident, shape);
-    k_lu_solve<TF, DIAG><<<grid, SOLVE_THREADS, smem, c->stream>>>(pool, perm, stride, m, count, x, z);
-    c->launched();
-}
+// One warp per block (dgh_kernels_solve.cuh).
 template <typename TF>
 void launch_solve(dgh_ctx *c, const TF *pool, const int *perm, size_t stride, int m, int count, const double *x,
-                  double *z, int shape = 0) {
-    if constexpr (sizeof(TF) == 4)
-        if (m < 64) return launch_solve_as<TF, true>(c, pool, perm, stride, m, count, x, z, shape);
-    launch_solve_as<TF, false>(c, pool, perm, stride, m, count, x, z, shape);
+                  double *z, int shape = 0, const float *scale = nullptr) {
+    const size_t smem = SOLVE_WARPS * solve_warp_bytes<TF>(m);
+    allow_dynamic_smem((const void *)k_lu_solve<TF>, smem);
+    int resident = 0;
+    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_lu_solve<TF>, SOLVE_THREADS, smem), "occupancy");
+    const int grid = solve_grid(c, count, SOLVE_WARPS, resident, shape);
+    k_lu_solve<TF><<<grid, SOLVE_THREADS, smem, c->stream>>>(pool, scale, perm, stride, m, count, x, z);
+    c->launched();
 }
-
 template <typename TF>
 void launch_solve_t(dgh_ctx *c, const TF *pool, const int *perm, size_t stride, int m, int count, const double *x,
                     double *z) {
-    constexpr int wpc = SOLVE_THREADS / 32;
-    const size_t smem = sizeof(TF) * (size_t)m * wpc;
-    const int want = (count + wpc - 1) / wpc;
+    const size_t smem = SOLVE_WARPS * solve_warp_bytes<TF, true>(m);
+    allow_dynamic_smem((const void *)k_lu_solve_t<TF>, smem);
     int resident = 0;
     ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_lu_solve_t<TF>, SOLVE_THREADS, smem), "occupancy");
-    const int grid = std::min(want, c->sms * std::max(1, resident));
+    const int grid = solve_grid(c, count, SOLVE_WARPS, resident, 0);
     k_lu_solve_t<TF><<<grid, SOLVE_THREADS, smem, c->stream>>>(pool, perm, stride, m, count, x, z);
-    c->launched();
-}
-
-// The DG cell blocks from their FP16 slabs (one warp per block, like launch_solve).
-void launch_solve_half(dgh_ctx *c, const double *x, double *z, int shape) {
-    constexpr int wpc = SOLVE_THREADS / 32;
-    const size_t smem = sizeof(float) * (size_t)pad8(c->m) * wpc;
-    int resident = 0;
-    ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_lu_solve_half, SOLVE_THREADS, smem), "occupancy");
-    const int grid = solve_grid(c, c->cells, wpc, resident, shape);
-    k_lu_solve_half<<<grid, SOLVE_THREADS, smem, c->stream>>>((const __half *)c->dg_pool, c->dg_scale, c->dg_perm, c->m,
-                                                               c->cells, x, z);
     c->launched();
 }
 
@@ -863,7 +855,9 @@ template <typename TF> void ilu2_apply(dgh_ctx *c, const double *x, double *z) {
 // The DG cell blocks' block-Jacobi solve z = M^{-1} x with grid shape `shape` (solve_grid).
 void dg_block_solve(dgh_ctx *c, int shape, const double *x, double *z) {
     const size_t stride = (size_t)c->m * c->m;
-    if (c->half16()) launch_solve_half(c, x, z, shape);
+    if (c->half16())
+        launch_solve<__half>(c, (const __half *)c->dg_pool, c->dg_perm, (size_t)c->m * pad8(c->m), c->m, c->cells, x, z, shape,
+                             c->dg_scale);
     else if (c->mixed()) launch_solve<float>(c, (const float *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z, shape);
     else launch_solve<double>(c, (const double *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z, shape);
 }
@@ -1260,16 +1254,11 @@ void gmres(dgh_ctx *c, int op, const double *rhs, double *x, int limit, double t
 void ls_solve_all(dgh_lockstep *L, int src, int dst, int j, int gate) {
     for (const auto &r : L->layouts) {
         if (r.key == 0)
-            k_ls_solve<double, false><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst,
-                                                                                     j, gate);
-        else if (r.key == 1)
-            k_ls_solve<float, false><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst,
-                                                                                    j, gate);
-        else if (r.key == 2)
-            k_ls_solve<float, true><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst,
-                                                                                   j, gate);
+            k_ls_solve<double><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
+        else if (r.key == 1 || r.key == 2)
+            k_ls_solve<float><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
         else if (r.key == 3)
-            k_ls_solve_half<<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
+            k_ls_solve<__half><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
         else
             k_ls_inv_apply<<<r.blocks, INV_APPLY_THREADS, 0, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
         L->launched();
@@ -1293,10 +1282,21 @@ void ls_jv_all(dgh_lockstep *L, int src, int dst, int gate) {
         L->launched(2);
     }
 }
+// A member's CTAs in a batched solve: no more than are resident, so that a warp's ring runs on from block
+// to block.
+int ls_solve_blocks(const dgh_ctx *c, int count) { return solve_grid(c, count, SOLVE_WARPS, 5, 0); }
+// Dynamic shared memory of the block solve of factor layout `key` (0 FP64, 1 and 2 FP32, 3 FP16).
+size_t ls_solve_smem(int key, int m) {
+    const size_t warp = key == 0 ? solve_warp_bytes<double>(m) : key == 3 ? solve_warp_bytes<__half>(m) : solve_warp_bytes<float>(m);
+    const void *fn = key == 0 ? (const void *)k_ls_solve<double>
+                     : key == 3 ? (const void *)k_ls_solve<__half>
+                                : (const void *)k_ls_solve<float>;
+    allow_dynamic_smem(fn, SOLVE_WARPS * warp);
+    return SOLVE_WARPS * warp;
+}
 // The HDG members' face-block Jacobi launches from their current state (FP32 inverses or LU
 // factors, chosen at each refresh): consecutive members with the same form share a launch.
 void ls_plan_face_precond(dgh_lockstep *L) {
-    constexpr int wpc = SOLVE_THREADS / 32;
     L->layouts.clear();
     std::vector<int> keys;
     for (int i = 0; i < (int)L->members.size(); ++i) {
@@ -1313,9 +1313,10 @@ void ls_plan_face_precond(dgh_lockstep *L) {
         L->host[i].solve0 = lr.blocks;
         L->host[i].pool = c->face_pool;
         L->host[i].perm = c->face_perm;
-        lr.blocks += (c->faces + wpc - 1) / wpc;
+        constexpr int inv_wpc = INV_APPLY_THREADS / 32;
+        lr.blocks += key == 4 ? (c->faces + inv_wpc - 1) / inv_wpc : ls_solve_blocks(c, c->faces);
         ++lr.count;
-        if (key != 4) lr.smem = std::max(lr.smem, (key == 0 ? sizeof(double) : sizeof(float)) * (size_t)c->fw * wpc);
+        if (key != 4) lr.smem = std::max(lr.smem, ls_solve_smem(key, c->fw));
     }
     if (keys != L->layout_keys && L->cycle) {  // a different launch plan: capture the cycle again
         ck(cudaGraphExecDestroy(L->cycle), "cudaGraphExecDestroy");
@@ -3412,7 +3413,6 @@ int dgh_lockstep_create_op(dgh_ctx *const *members, int count, int op, dgh_locks
             ck(cudaMallocHost(&L->host, sizeof(LsMember) * count), "cudaMallocHost");
             ck(cudaMallocHost(&L->flags_host, sizeof(int) * count), "cudaMallocHost");
             ck(cudaMallocHost(&L->tails_host, sizeof(LsTail) * count), "cudaMallocHost");
-            constexpr int wpc = SOLVE_THREADS / 32;
             auto layout_of = [&](const dgh_ctx *c) { return c->half16() ? 3 : !c->mixed() ? 0 : c->m < 64 ? 2 : 1; };
             for (int i = 0; i < count; ++i) {
                 dgh_ctx *c = L->members[i];
@@ -3437,7 +3437,7 @@ int dgh_lockstep_create_op(dgh_ctx *const *members, int count, int op, dgh_locks
                 t.pool = c->dg_pool;
                 t.scale = c->dg_scale;
                 t.perm = c->dg_perm;
-                t.stride = (size_t)c->m * c->m;
+                t.stride = (size_t)c->m * (c->half16() ? pad8(c->m) : c->m);
                 t.m = c->m;
                 t.cells = c->cells;
                 t.traces = c->traces2;
@@ -3478,10 +3478,9 @@ int dgh_lockstep_create_op(dgh_ctx *const *members, int count, int op, dgh_locks
                 }
                 auto &lr = L->layouts.back();
                 t.solve0 = lr.blocks;
-                lr.blocks += (c->cells + wpc - 1) / wpc;
+                lr.blocks += ls_solve_blocks(c, c->cells);
                 ++lr.count;
-                const size_t row = key == 3 ? sizeof(float) * pad8(c->m) : (key == 0 ? sizeof(double) : sizeof(float)) * c->m;
-                lr.smem = std::max(lr.smem, row * wpc);
+                lr.smem = std::max(lr.smem, ls_solve_smem(key, c->m));
             }
             for (const auto &r : L->layouts)
                 for (const auto &q : L->layouts)

@@ -10,7 +10,7 @@
 #include "dgh_kernels_dg.cuh"
 #include "dgh_kernels_hdg.cuh"
 #include "dgh_kernels_krylov.cuh"
-#include "dgh_kernels_lu.cuh"
+#include "dgh_kernels_solve.cuh"
 
 namespace dgh {
 
@@ -160,27 +160,17 @@ __global__ void k_ls_tails(const LsMember *t, int count, LsTail *out) {
 }
 
 // ---- block-Jacobi solve z = M^{-1} src over the members [first, first + count) of one layout ----
-// The solve bodies keep the compiler's own FMA choices (they pair FP32 operations and are
-// faster than any explicitly rounded form); that they compute the same bits here as in
-// k_lu_solve / k_lu_solve_half is checked by the lockstep tests, member by member.
-template <typename T, bool DIAG>
-__global__ void __launch_bounds__(SOLVE_THREADS, (solve_min_blocks<T, DIAG>()))
+// The solve body rounds every product and sum in a stated order, so it computes the same bits here as
+// in k_lu_solve.
+template <typename T>
+__global__ void __launch_bounds__(SOLVE_THREADS, SOLVE_CTAS<T>)
 k_ls_solve(const LsMember *t, int first, int count, int src, int dst, int j, int gate) {
     const int i = ls_find(t, first, count, blockIdx.x, LS_SOLVE);
     const LsMember &a = t[i];
     if (!ls_on(a, gate)) return;
     const int blocks = (i + 1 < first + count ? t[i + 1].solve0 : gridDim.x) - a.solve0;
-    lu_solve_body<T, DIAG>(blockIdx.x - a.solve0, blocks, (const T *)a.pool, a.perm, a.stride, a.m, a.cells,
-                           ls_vec(a, src, j), ls_vec(a, dst, j));
-}
-__global__ void __launch_bounds__(SOLVE_THREADS, 5)
-k_ls_solve_half(const LsMember *t, int first, int count, int src, int dst, int j, int gate) {
-    const int i = ls_find(t, first, count, blockIdx.x, LS_SOLVE);
-    const LsMember &a = t[i];
-    if (!ls_on(a, gate)) return;
-    const int blocks = (i + 1 < first + count ? t[i + 1].solve0 : gridDim.x) - a.solve0;
-    lu_solve_half_body(blockIdx.x - a.solve0, blocks, (const __half *)a.pool, a.scale, a.perm, a.m, a.cells,
-                       ls_vec(a, src, j), ls_vec(a, dst, j));
+    lu_solve_body<T>(blockIdx.x - a.solve0, blocks, (const T *)a.pool, a.scale, a.perm, a.stride, a.m, a.cells,
+                     ls_vec(a, src, j), ls_vec(a, dst, j));
 }
 
 // ---- face-block Jacobi of HDG members from FP32 inverses (k_inv_apply's body) ----------------

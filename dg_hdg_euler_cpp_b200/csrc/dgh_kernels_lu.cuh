@@ -576,126 +576,6 @@ k_inv_apply(const float *__restrict__ inv, int m, int count, const double *__res
     inv_apply_body(blockIdx.x, gridDim.x, inv, m, count, rhs, z);
 }
 
-// Block solve z = A^{-1} b with the factors of k_lu (block_jacobi.hpp:24-39): permute, unit
-// lower solve, upper solve.  One warp owns one block and streams its factors exactly once with
-// no CTA-wide barriers; lane i owns row 32 s + i of slab s and reads 16-byte column groups of
-// the slab layout above.  Off-diagonal parts are per-lane dot products (four 16-byte loads in
-// flight per lane, four accumulators); the diagonal triangles of the 32-row slabs are solved with
-// warp shuffles.  T is the factor and arithmetic precision (FP32 factors accumulate in FP32);
-// b and z are FP64.  The forward and backward sweeps share one loop body, which keeps the
-// kernel at <= 48 registers (FP32; five 256-thread CTAs per SM) or 64 (FP64).  DIAG loads a full
-// slab's diagonal row into registers before its triangle (all its loads in flight at once): the
-// FP32 form for narrow blocks (the HDG face blocks, m = 4n), whose time is mostly triangles.
-constexpr int SOLVE_THREADS = 256;
-template <typename T, bool DIAG> constexpr int solve_min_blocks() { return sizeof(T) == 4 && !DIAG ? 5 : 4; }
-// The body takes its block index bx and block count G explicitly (the batched solve of a
-// lockstep batch runs it over each member's blocks).
-template <typename T, bool DIAG>
-__device__ __forceinline__ void lu_solve_body(int bx, int G, const T *__restrict__ pool, const int *__restrict__ perm,
-                                              size_t stride, int m, int count, const double *__restrict__ rhs,
-                                              double *__restrict__ z) {
-    using SV = SlabVec<T>;
-    using V = typename SV::V;
-    constexpr int W = SV::W, ND = 32 / W;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    T *y = reinterpret_cast<T *>(smraw) + (size_t)wib * m;
-    // m * sizeof(T) is a multiple of 16 (m = 4n^2 or 4n), so every warp's y is 16-byte aligned
-    const V *yv = reinterpret_cast<const V *>(y);
-    const int warps = G * (SOLVE_THREADS / 32);
-    const int slabs = (m + 31) / 32;
-    for (int blk = bx * (SOLVE_THREADS / 32) + wib; blk < count; blk += warps) {
-        const T *A = pool + (size_t)blk * stride;
-        const int *pm = perm + (size_t)blk * m;
-        const double *b = rhs + (size_t)blk * m;
-        for (int i = lane; i < m; i += 32) y[i] = (T)b[pm[i]];
-        __syncwarp();
-        // dir 0: forward, L y = P b (slabs in order, columns left of the slab); dir 1: backward,
-        // U z = y (slabs in reverse, columns right of the slab)
-        for (int dir = 0; dir < 2; ++dir) {
-            for (int si = 0; si < slabs; ++si) {
-                const int s = dir == 0 ? si : slabs - 1 - si;
-                const int r0 = 32 * s, nt = min(32, m - r0), hi = r0 + nt;
-                const T *S = A + (size_t)r0 * m;
-                const V *Sv = reinterpret_cast<const V *>(S);
-                const bool act = lane < nt;
-                T acc0 = 0, acc1 = 0, acc2 = 0, acc3 = 0;
-                if (act) {
-                    const int g1 = dir == 0 ? r0 / W : m / W;
-                    int g = dir == 0 ? 0 : hi / W;
-                    for (; g + 4 <= g1; g += 4) {  // four independent 16-byte loads in flight per lane
-                        const V a0 = Sv[(size_t)g * nt + lane], a1 = Sv[(size_t)(g + 1) * nt + lane];
-                        const V a2 = Sv[(size_t)(g + 2) * nt + lane], a3 = Sv[(size_t)(g + 3) * nt + lane];
-                        acc0 += SV::dotv(a0, yv[g]);
-                        acc1 += SV::dotv(a1, yv[g + 1]);
-                        acc2 += SV::dotv(a2, yv[g + 2]);
-                        acc3 += SV::dotv(a3, yv[g + 3]);
-                    }
-                    for (; g < g1; ++g) acc0 += SV::dotv(Sv[(size_t)g * nt + lane], yv[g]);
-                }
-                T t = act ? y[r0 + lane] - ((acc0 + acc1) + (acc2 + acc3)) : T(0);
-                if (DIAG && nt == 32) {
-                    V d[ND];
-#pragma unroll
-                    for (int q = 0; q < ND; ++q) d[q] = Sv[(size_t)(r0 / W + q) * 32 + lane];
-                    if (dir == 0) {
-#pragma unroll
-                        for (int q = 0; q < ND; ++q) {
-                            const T *e = reinterpret_cast<const T *>(&d[q]);
-#pragma unroll
-                            for (int w = 0; w < W; ++w) {
-                                const int jj = W * q + w;
-                                const T l = lane > jj ? e[w] : T(0);
-                                const T yj = __shfl_sync(0xffffffffu, t, jj);
-                                t -= l * yj;
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int q = ND - 1; q >= 0; --q) {
-                            const T *e = reinterpret_cast<const T *>(&d[q]);
-#pragma unroll
-                            for (int w = W - 1; w >= 0; --w) {
-                                const int jj = W * q + w;
-                                const T u = e[w];
-                                if (lane == jj) t = t / u;
-                                const T yj = __shfl_sync(0xffffffffu, t, jj);
-                                if (lane < jj) t -= u * yj;
-                            }
-                        }
-                    }
-                } else if (dir == 0) {
-                    for (int jj = 0; jj < nt; ++jj) {
-                        const T l = (act && lane > jj) ? S[slab_at<T>(nt, lane, r0 + jj)] : T(0);
-                        const T yj = __shfl_sync(0xffffffffu, t, jj);
-                        t -= l * yj;
-                    }
-                } else {
-                    for (int jj = nt - 1; jj >= 0; --jj) {
-                        // row `lane` uses U(lane, jj) only on and right of its diagonal: the
-                        // lower half of the diagonal block was read by the forward sweep and is
-                        // not fetched again
-                        const T u = (act && lane <= jj) ? S[slab_at<T>(nt, lane, r0 + jj)] : T(1);
-                        if (lane == jj) t = t / u;
-                        const T yj = __shfl_sync(0xffffffffu, t, jj);
-                        if (lane < jj) t -= u * yj;
-                    }
-                }
-                if (act) y[r0 + lane] = t;
-                __syncwarp();
-            }
-        }
-        for (int i = lane; i < m; i += 32) z[(size_t)blk * m + i] = (double)y[i];
-        __syncwarp();
-    }
-}
-template <typename T, bool DIAG>
-__global__ void __launch_bounds__(SOLVE_THREADS, (solve_min_blocks<T, DIAG>()))
-k_lu_solve(const T *__restrict__ pool, const int *__restrict__ perm, size_t stride, int m, int count,
-           const double *__restrict__ rhs, double *__restrict__ z) {
-    lu_solve_body<T, DIAG>(blockIdx.x, gridDim.x, pool, perm, stride, m, count, rhs, z);
-}
-
 // Packs row-major factored FP64 blocks (LU in place, row length m, rows in position order) into
 // the FP16 slabs and row scales: one warp per 32-row slab of a block, lane i owning row 32 s + i.
 __global__ void k_pack_half(const double *__restrict__ src, int m, int count, __half *__restrict__ dst,
@@ -721,189 +601,6 @@ __global__ void k_pack_half(const double *__restrict__ src, int m, int count, __
             v[w] = __double2half(j >= row ? a * inv : a);
         }
         *reinterpret_cast<uint4 *>(out + (size_t)g * nt * H_W + lane * H_W) = *reinterpret_cast<const uint4 *>(v);
-    }
-}
-
-// z = A^{-1} b per block from the FP16 slabs: k_lu_solve's structure (one warp per block, lane
-// i owns row 32 s + i, four 16-byte loads in flight, shuffled diagonal triangles) with FP32
-// arithmetic; the backward sweep multiplies each row's right-hand side by its row scale.
-__device__ __forceinline__ void lu_solve_half_body(int bx, int G, const __half *__restrict__ pool,
-                                                   const float *__restrict__ row_scale, const int *__restrict__ perm,
-                                                   int m, int count, const double *__restrict__ rhs,
-                                                   double *__restrict__ z) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int mp = pad8(m), lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    float *y = reinterpret_cast<float *>(smraw) + (size_t)wib * mp;
-    const float4 *yv = reinterpret_cast<const float4 *>(y);
-    const int warps = G * (SOLVE_THREADS / 32);
-    const int slabs = (m + 31) / 32;
-    auto dot8 = [&](const uint4 &a, int g) {
-        const __half2 *h = reinterpret_cast<const __half2 *>(&a);
-        const float4 y0 = yv[2 * g], y1 = yv[2 * g + 1];
-        const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]);
-        const float2 f2 = __half22float2(h[2]), f3 = __half22float2(h[3]);
-        return (f0.x * y0.x + f0.y * y0.y) + (f1.x * y0.z + f1.y * y0.w) + (f2.x * y1.x + f2.y * y1.y) +
-               (f3.x * y1.z + f3.y * y1.w);
-    };
-    for (int blk = bx * (SOLVE_THREADS / 32) + wib; blk < count; blk += warps) {
-        const __half *A = pool + (size_t)blk * m * mp;
-        const int *pm = perm + (size_t)blk * m;
-        const float *rs = row_scale + (size_t)blk * m;
-        const double *b = rhs + (size_t)blk * m;
-        for (int i = lane; i < mp; i += 32) y[i] = i < m ? (float)b[pm[i]] : 0.f;
-        __syncwarp();
-        for (int dir = 0; dir < 2; ++dir) {
-            for (int si = 0; si < slabs; ++si) {
-                const int s = dir == 0 ? si : slabs - 1 - si;
-                const int r0 = 32 * s, nt = min(32, m - r0), hi = r0 + nt;
-                const __half *S = A + (size_t)r0 * mp;
-                const uint4 *Sv = reinterpret_cast<const uint4 *>(S);
-                const bool act = lane < nt;
-                float acc0 = 0, acc1 = 0, acc2 = 0, acc3 = 0;
-                if (act) {
-                    // forward: the groups left of the slab; backward: the groups right of it (the
-                    // last slab, whose end may fall inside a group, has none)
-                    const int g1 = dir == 0 ? r0 / H_W : mp / H_W;
-                    int g = dir == 0 ? 0 : (hi >= m ? mp / H_W : hi / H_W);
-                    for (; g + 4 <= g1; g += 4) {
-                        const uint4 a0 = Sv[(size_t)g * nt + lane], a1 = Sv[(size_t)(g + 1) * nt + lane];
-                        const uint4 a2 = Sv[(size_t)(g + 2) * nt + lane], a3 = Sv[(size_t)(g + 3) * nt + lane];
-                        acc0 += dot8(a0, g);
-                        acc1 += dot8(a1, g + 1);
-                        acc2 += dot8(a2, g + 2);
-                        acc3 += dot8(a3, g + 3);
-                    }
-                    for (; g < g1; ++g) acc0 += dot8(Sv[(size_t)g * nt + lane], g);
-                }
-                // the slab's diagonal 32 x 32 block: this lane's row, four 16-byte groups loaded at
-                // once (r0 is a multiple of 32, so the block starts a group)
-                uint4 dg[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    dg[q] = (act && 8 * q < nt) ? Sv[(size_t)(r0 / H_W + q) * nt + lane] : make_uint4(0, 0, 0, 0);
-                float t = 0.f;
-                if (act) t = (dir == 0 ? y[r0 + lane] : y[r0 + lane] * rs[r0 + lane]) - ((acc0 + acc1) + (acc2 + acc3));
-                auto at = [&](int jj) {  // stored entry (row r0 + lane, column r0 + jj), jj a constant
-                    const uint4 &v = dg[jj >> 3];
-                    const int w = (jj >> 1) & 3;
-                    const unsigned word = w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w;
-                    return __half2float(__ushort_as_half((unsigned short)((jj & 1) ? word >> 16 : word & 0xffffu)));
-                };
-                if (dir == 0) {
-#pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
-                        if (jj >= nt) break;
-                        const float l = lane > jj ? at(jj) : 0.f;
-                        const float yj = __shfl_sync(0xffffffffu, t, jj);
-                        t -= l * yj;
-                    }
-                } else {
-#pragma unroll
-                    for (int jj = 31; jj >= 0; --jj) {
-                        if (jj >= nt) continue;
-                        const float u = lane <= jj ? at(jj) : 1.f;
-                        if (lane == jj) t = t / u;
-                        const float yj = __shfl_sync(0xffffffffu, t, jj);
-                        if (lane < jj) t -= u * yj;
-                    }
-                }
-                if (act) y[r0 + lane] = t;
-                __syncwarp();
-            }
-        }
-        for (int i = lane; i < m; i += 32) z[(size_t)blk * m + i] = (double)y[i];
-        __syncwarp();
-    }
-}
-__global__ void __launch_bounds__(SOLVE_THREADS, 5)
-k_lu_solve_half(const __half *__restrict__ pool, const float *__restrict__ row_scale, const int *__restrict__ perm,
-                int m, int count, const double *__restrict__ rhs, double *__restrict__ z) {
-    lu_solve_half_body(blockIdx.x, gridDim.x, pool, row_scale, perm, m, count, rhs, z);
-}
-
-// Transposed block solve z = A^{-T} b with the same slab-layout factors (A = P^T L U, so
-// A^{-T} b = P^T L^{-T} U^{-T} b): a forward solve with U^T (lower, with U's diagonal), a
-// backward solve with L^T (unit upper), then the scatter z[perm[i]] = x[i].  Slab s holds rows
-// 32s.. of U and L; once a slab's unknowns are final, its rows are applied to the remaining
-// unknowns with each lane owning one 16-byte column group (no CTA barriers, one warp per block).
-template <typename T>
-__global__ void __launch_bounds__(SOLVE_THREADS)
-k_lu_solve_t(const T *__restrict__ pool, const int *__restrict__ perm, size_t stride, int m, int count,
-             const double *__restrict__ rhs, double *__restrict__ z) {
-    using SV = SlabVec<T>;
-    using V = typename SV::V;
-    constexpr int W = SV::W;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    T *y = reinterpret_cast<T *>(smraw) + (size_t)wib * m;
-    const int warps = gridDim.x * (SOLVE_THREADS / 32);
-    const int slabs = (m + 31) / 32;
-    for (int blk = blockIdx.x * (SOLVE_THREADS / 32) + wib; blk < count; blk += warps) {
-        const T *A = pool + (size_t)blk * stride;
-        const int *pm = perm + (size_t)blk * m;
-        const double *b = rhs + (size_t)blk * m;
-        for (int i = lane; i < m; i += 32) y[i] = (T)b[i];
-        __syncwarp();
-        // U^T y = b, forward by slabs
-        for (int s = 0; s < slabs; ++s) {
-            const int r0 = 32 * s, nt = min(32, m - r0), hi = r0 + nt;
-            const T *S = A + (size_t)r0 * m;
-            T t = lane < nt ? y[r0 + lane] : T(0);
-            for (int jj = 0; jj < nt; ++jj) {
-                const T d = lane == jj ? S[slab_at<T>(nt, jj, r0 + jj)] : T(1);
-                if (lane == jj) t = t / d;
-                const T yj = __shfl_sync(0xffffffffu, t, jj);
-                // U^T[r0+lane][r0+jj] = U[r0+jj][r0+lane], nonzero for lane > jj
-                if (lane > jj && lane < nt) t -= S[slab_at<T>(nt, jj, r0 + lane)] * yj;
-            }
-            if (lane < nt) y[r0 + lane] = t;
-            __syncwarp();
-            for (int g = hi / W + lane; g < m / W; g += 32) {
-                T acc[W];
-#pragma unroll
-                for (int e = 0; e < W; ++e) acc[e] = 0;
-                for (int i = 0; i < nt; ++i) {
-                    const V v = reinterpret_cast<const V *>(S)[(size_t)g * nt + i];
-                    const T yi = y[r0 + i];
-                    const T *vv = reinterpret_cast<const T *>(&v);
-#pragma unroll
-                    for (int e = 0; e < W; ++e) acc[e] += vv[e] * yi;
-                }
-#pragma unroll
-                for (int e = 0; e < W; ++e) y[g * W + e] -= acc[e];
-            }
-            __syncwarp();
-        }
-        // L^T x = y (unit upper), backward by slabs
-        for (int s = slabs - 1; s >= 0; --s) {
-            const int r0 = 32 * s, nt = min(32, m - r0);
-            const T *S = A + (size_t)r0 * m;
-            T t = lane < nt ? y[r0 + lane] : T(0);
-            for (int jj = nt - 1; jj >= 0; --jj) {
-                const T yj = __shfl_sync(0xffffffffu, t, jj);
-                // L^T[r0+lane][r0+jj] = L[r0+jj][r0+lane], nonzero for lane < jj
-                if (lane < jj) t -= S[slab_at<T>(nt, jj, r0 + lane)] * yj;
-            }
-            if (lane < nt) y[r0 + lane] = t;
-            __syncwarp();
-            for (int g = lane; g < r0 / W; g += 32) {
-                T acc[W];
-#pragma unroll
-                for (int e = 0; e < W; ++e) acc[e] = 0;
-                for (int i = 0; i < nt; ++i) {
-                    const V v = reinterpret_cast<const V *>(S)[(size_t)g * nt + i];
-                    const T yi = y[r0 + i];
-                    const T *vv = reinterpret_cast<const T *>(&v);
-#pragma unroll
-                    for (int e = 0; e < W; ++e) acc[e] += vv[e] * yi;
-                }
-#pragma unroll
-                for (int e = 0; e < W; ++e) y[g * W + e] -= acc[e];
-            }
-            __syncwarp();
-        }
-        for (int i = lane; i < m; i += 32) z[(size_t)blk * m + pm[i]] = (double)y[i];
-        __syncwarp();
     }
 }
 
