@@ -281,6 +281,13 @@ struct dgh_ctx {
     bool has_dg() const { return cfg.method == DGH_METHOD_DG || cfg.method == DGH_METHOD_BOTH; }
     bool has_hdg() const { return cfg.method == DGH_METHOD_HDG || cfg.method == DGH_METHOD_BOTH; }
     int team_blocks(int cpb) const { return (cells + cpb - 1) / cpb; }
+    // The sweeps' CTAs: RED_BLOCKS_PER_SM on every SM, or at small sizes a pair of elements per thread (a CTA
+    // without elements would still add partial sums for the reductions to read).  147,456 unknowns: 288 CTAs, a
+    // sweep of 14 vectors 6.8 us; 592 CTAs, 10.7.
+    void size_sweeps() {
+        const long long pairs = (std::max(N, NT) + 1) / 2;
+        red_grid = (int)std::min<long long>(red_grid, std::max<long long>(1, (pairs + KR_THREADS - 1) / KR_THREADS));
+    }
     // Deterministic weighted reduction helpers (return host values).
     // interior: x is a volume vector whose ghost rows a slab must skip (otherwise its ghost rows
     // or faces are zero)
@@ -1033,14 +1040,23 @@ void maxpy_dot(dgh_ctx *c, const double *V, size_t ld, int K, const double *h, d
     c->launched(2);
     slab_sum(c, out, K);
 }
+// The last sweep of step K - 1, with the update of the Hessenberg column and the continue flag (once a
+// slab's norm has been added over its ranks).
 void maxpy_norm(dgh_ctx *c, const double *V, size_t ld, int K, const double *h, double *x, const double *W, long long n,
-                double *out) {
+                cudaGraphConditionalHandle handle, int use_h) {
 #define C_(NV) maxpy_t<NV, 1>(c, V, ld, K, h, x, W, n)
     DGH_DISPATCH_K(K, C_);
 #undef C_
-    k_reduce<<<1, KR_THREADS, 0, c->stream>>>(c->partial, c->red_grid, out);
     c->launched(2);
-    slab_sum(c, out, 1);
+    if (!c->slabbed()) {
+        k_reduce_update<<<1, KR_THREADS, 0, c->stream>>>(c->partial, c->red_grid, c->red, c->gdev, K - 1, handle, use_h);
+        return;
+    }
+    double *norm2 = c->red + 2 * KR_MAXK;
+    k_reduce<<<1, KR_THREADS, 0, c->stream>>>(c->partial, c->red_grid, norm2);
+    slab_sum(c, norm2, 1);
+    k_gmres_update<<<1, 32, 0, c->stream>>>(c->gdev, c->red, K - 1, handle, use_h);
+    c->launched();
 }
 void lincomb(dgh_ctx *c, const double *V, size_t ld, int K, const double *coef, double *out, long long n) {
 #define C_(NV) lincomb_t<NV>(c, V, ld, K, coef, out, n)
@@ -1055,7 +1071,7 @@ void axpby(dgh_ctx *c, double a, const double *x, double b, const double *y, dou
 
 // gmres.cpp:17-86 with the CGS2 passes fused as dot | axpy+dot | axpy+norm.  One restart cycle
 // is three segments: start (beta, V0 = r / beta, k_gmres_init), up to `restart` Arnoldi steps
-// (preconditioner, operator, three sweeps, normalisation, k_gmres_update), and finish (back
+// (preconditioner, operator, three sweeps, the last with the update, normalisation), and finish (back
 // substitution, x += M^{-1} V y, true residual and its norm).  The cycle is either launched step
 // by step (the host reads the device's continue flag after every step) or replayed as one CUDA
 // graph whose steps are conditional nodes; the kernels and hence the numbers are the same.
@@ -1086,12 +1102,10 @@ int gmres_step(dgh_ctx *c, const GmresCall &g, int j, cudaGraphConditionalHandle
         Timed tm(c, DGH_TIMER_ARNOLDI);
         mdot(c, V, ld, j + 1, w, g.W, g.n, h1);
         maxpy_dot(c, V, ld, j + 1, h1, w, g.W, g.n, h2);
-        maxpy_norm(c, V, ld, j + 1, h2, w, g.W, g.n, nrm);
+        maxpy_norm(c, V, ld, j + 1, h2, w, g.W, g.n, h, use_h);
         k_scale_div<<<c->red_grid, KR_THREADS, 0, c->stream>>>(w, nrm, 1, V + (size_t)(j + 1) * ld, g.n);
         c->launched();
     }
-    k_gmres_update<<<1, 32, 0, c->stream>>>(c->gdev, c->red, j, h, use_h);
-    c->launched();
     return (int)(c->launches - before);
 }
 int gmres_finish(dgh_ctx *c, const GmresCall &g) {
@@ -1355,10 +1369,9 @@ int ls_seg_step(dgh_lockstep *L, cudaStream_t st, int j) {
 #define C_(NV) k_ls_maxpy<NV, 1><<<L->red_total, KR_THREADS, 0, st>>>(L->table, cnt, K)
     DGH_DISPATCH_K(K, C_);
 #undef C_
-    k_ls_reduce<<<cnt, KR_THREADS, 0, st>>>(L->table, cnt, 1, 2, 1);
+    k_ls_reduce_update<<<cnt, KR_THREADS, 0, st>>>(L->table, j);
     k_ls_scale_div<<<L->red_total, KR_THREADS, 0, st>>>(L->table, cnt, LS_W, LS_VJ1, j, 1);
-    k_ls_gmres_update<<<cnt, 32, 0, st>>>(L->table, j);
-    L->launched(8);
+    L->launched(7);
     return (int)(L->launches - before);
 }
 int ls_seg_finish(dgh_lockstep *L, cudaStream_t st) {
@@ -1757,6 +1770,7 @@ void create1(dgh_ctx *c, const dgh_config &k) {
     c->speeds = c->alloc<double>(c->nspeeds);
     c->traces = c->alloc<double>((size_t)c->cells * T1);
     c->traces2 = c->alloc<double>((size_t)c->cells * T1);
+    c->size_sweeps();
     c->partial = c->alloc<double>((size_t)std::max<long long>(KR_MAXK * c->red_grid, 4LL * c->cells + 64));
     c->red = c->alloc<double>(4 * KR_MAXK);
     c->vol = c->alloc<double>((size_t)c->cells * Q * 9);
@@ -2002,7 +2016,8 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
         c->speeds = c->alloc<double>(2 * (size_t)c->faces * n);
         c->traces = c->alloc<double>((size_t)c->cells * NFACES * n * NVAR);
         c->traces2 = c->alloc<double>((size_t)c->cells * NFACES * n * NVAR);
-        c->partial = c->alloc<double>((size_t)std::max<long long>(KR_MAXK * c->red_grid, 4LL * c->cells + 64));
+        c->size_sweeps();
+    c->partial = c->alloc<double>((size_t)std::max<long long>(KR_MAXK * c->red_grid, 4LL * c->cells + 64));
         c->red = c->alloc<double>(4 * KR_MAXK);
         c->vol = c->alloc<double>((size_t)c->cells * c->P * 3);
         c->fcache = c->alloc<double>((size_t)c->faces * n * 8);

@@ -246,8 +246,8 @@ k_rho2(const double *__restrict__ u, const double *__restrict__ mass, int plane,
 }
 
 // ---- Device-resident GMRES control (gmres.cpp:24-86): the Hessenberg column, the Givens
-// rotations, the inner-loop break and the least-squares back substitution run in one-thread
-// kernels, so a whole restart cycle can be replayed as one CUDA graph whose Arnoldi steps are
+// rotations, the inner-loop break and the least-squares back substitution run on one warp (its lane 0
+// where a chain has to be followed), so a whole restart cycle can be replayed as one CUDA graph whose Arnoldi steps are
 // conditional nodes (the break of gmres.cpp:65-67 sets the condition to zero).  The same kernels
 // run when the cycle is launched step by step, so both ways give the same numbers.  Each step's
 // conditional node has its own handle, set by the kernel that precedes the step.
@@ -258,80 +258,113 @@ struct GmresDev {
     int iters, limit, count, cont, status, restart;
 };
 
+// The bodies below are called by one whole warp.
 // Cycle start: beta = ||r|| (from the reduction at nrm2), g = beta e_1, and whether to iterate
 // (gmres.cpp:25-27 and the loop condition of :33).
 __device__ __forceinline__ int gmres_init_body(GmresDev *d, const double *nrm2) {
+    const int lane = threadIdx.x & 31;
     const double beta = sqrt(fmax(0., *nrm2));
-    d->beta = beta;
-    for (int i = 0; i < (KR_MAXK + 1) * KR_MAXK; ++i) d->H[i] = 0.;
-    for (int i = 0; i <= KR_MAXK; ++i) d->g[i] = 0.;
-    d->g[0] = beta;
-    d->count = 0;
+    for (int i = lane; i < (KR_MAXK + 1) * KR_MAXK; i += 32) d->H[i] = 0.;
+    for (int i = lane; i <= KR_MAXK; i += 32) d->g[i] = i == 0 ? beta : 0.;
     const int cont = !(beta <= d->tol * d->rhs_norm) && d->restart > 0 && d->iters < d->limit;
-    d->cont = cont;
+    if (lane == 0) {
+        d->beta = beta;
+        d->count = 0;
+        d->cont = cont;
+    }
     return cont;
 }
 __global__ void k_gmres_init(GmresDev *d, const double *nrm2, cudaGraphConditionalHandle h, int use_h) {
-    if (threadIdx.x != 0) return;
     const int cont = gmres_init_body(d, nrm2);
-    if (use_h) cudaGraphSetConditional(h, cont);
+    if (use_h && threadIdx.x == 0) cudaGraphSetConditional(h, cont);
 }
 
 // After the CGS2 sweeps of step j: column j of H from the two projections (red[0..j],
 // red[KR_MAXK..]) and the norm (red[2 KR_MAXK]), the earlier rotations, the new rotation, the
 // rotated right-hand side and the break test (gmres.cpp:42-67).  In a captured cycle h is the
-// handle of step j+1's conditional node.
+// handle of step j+1's conditional node.  The lanes fetch the column and the rotations at once; lane 0
+// follows the chain of rotations in shared memory.  Returns lane 0's continue flag.
 __device__ __forceinline__ int gmres_update_body(GmresDev *d, const double *red, int j) {
     constexpr int LDH = KR_MAXK + 1;
+    __shared__ double h[LDH], cs[KR_MAXK], sn[KR_MAXK];
+    const int lane = threadIdx.x & 31;
     double *H = d->H + (size_t)j * LDH;
-    for (int i = 0; i <= j; ++i) H[i] = (0. + red[i]) + red[KR_MAXK + i];
-    const double next = sqrt(fmax(0., red[2 * KR_MAXK]));
-    H[j + 1] = next;
-    for (int i = 0; i < j; ++i) {
-        const double a = H[i], b = H[i + 1];
-        H[i] = rfma(d->cs[i], a, rmul(d->sn[i], b));
-        H[i + 1] = rfma(-d->sn[i], a, rmul(d->cs[i], b));
+    if (lane <= j) h[lane] = radd(radd(0., red[lane]), red[KR_MAXK + lane]);
+    if (lane < j) {
+        cs[lane] = d->cs[lane];
+        sn[lane] = d->sn[lane];
     }
-    const double dd = hypot(H[j], H[j + 1]);
-    if (!(isfinite(dd) && dd > 0)) {  // "GMRES Arnoldi breakdown", reported by the host
-        d->status = 1;
-        d->cont = 0;
-        return 0;
+    __syncwarp();
+    int cont = 0;
+    if (lane == 0) {
+        const double next = sqrt(fmax(0., red[2 * KR_MAXK])), gj = d->g[j];
+        double a = h[0];
+        for (int i = 0; i < j; ++i) {
+            const double b = h[i + 1];
+            h[i] = rfma(cs[i], a, rmul(sn[i], b));
+            a = rfma(-sn[i], a, rmul(cs[i], b));
+        }
+        const double dd = hypot(a, next);
+        h[j] = dd;
+        if (!(isfinite(dd) && dd > 0)) {  // "GMRES Arnoldi breakdown", reported by the host
+            d->status = 1;
+        } else {
+            const double c = a / dd, sj = next / dd, gn = -sj * gj;
+            d->cs[j] = c;
+            d->sn[j] = sj;
+            d->g[j + 1] = gn;
+            d->g[j] = gj * c;
+            d->iters += 1;
+            d->count = j + 1;
+            cont = !(fabs(gn) <= d->tol * d->rhs_norm || next <= 2.2250738585072014e-308) && j + 1 < d->restart &&
+                   d->iters < d->limit;
+        }
+        d->cont = cont;
     }
-    d->cs[j] = H[j] / dd;
-    d->sn[j] = H[j + 1] / dd;
-    H[j] = dd;
-    H[j + 1] = 0;
-    d->g[j + 1] = -d->sn[j] * d->g[j];
-    d->g[j] *= d->cs[j];
-    d->iters += 1;
-    d->count = j + 1;
-    const int cont = !(fabs(d->g[j + 1]) <= d->tol * d->rhs_norm || next <= 2.2250738585072014e-308) &&
-                     j + 1 < d->restart && d->iters < d->limit;
-    d->cont = cont;
+    __syncwarp();
+    if (lane <= j) H[lane] = h[lane];
+    if (lane == 0) H[j + 1] = 0;
     return cont;
 }
-__global__ void k_gmres_update(GmresDev *d, const double *red, int j, cudaGraphConditionalHandle h, int use_h) {
-    if (threadIdx.x != 0) return;
+// The norm's reduction (k_reduce of one entry) and, with it, the update of step j: one launch of 3.3 us at
+// 4,096 cells of degree 2 (4.4 us at 20 basis vectors) in place of two of 2.5 and 4.8 us, the second of one
+// thread whose loads came one after the other.  (Letting the last CTA of a sweep do its reduction saved
+// three more launches and lost 15 to 20 us a sweep: one SM reads all of the partial sums.)
+__global__ void __launch_bounds__(KR_THREADS)
+k_reduce_update(const double *__restrict__ partial, int G, double *red, GmresDev *d, int j, cudaGraphConditionalHandle h,
+                int use_h) {
+    reduce_body(0, partial, G, red + 2 * KR_MAXK);
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
     const int cont = gmres_update_body(d, red, j);
-    if (use_h) cudaGraphSetConditional(h, cont);
+    if (use_h && threadIdx.x == 0) cudaGraphSetConditional(h, cont);
+}
+__global__ void k_gmres_update(GmresDev *d, const double *red, int j, cudaGraphConditionalHandle h, int use_h) {
+    const int cont = gmres_update_body(d, red, j);
+    if (use_h && threadIdx.x == 0) cudaGraphSetConditional(h, cont);
 }
 
-// y = H(0:count, 0:count)^{-1} g (gmres.cpp:69-74); coef = y padded with zeros.
+// y = H(0:count, 0:count)^{-1} g (gmres.cpp:69-74); coef = y padded with zeros.  Lane i holds row i.
 __device__ __forceinline__ void gmres_backsolve_body(GmresDev *d, double *coef) {
     constexpr int LDH = KR_MAXK + 1;
-    const int cnt = d->count;
-    for (int i = cnt - 1; i >= 0; --i) {
-        double value = d->g[i];
-        for (int jj = i + 1; jj < cnt; ++jj) value = rfma(-d->H[(size_t)jj * LDH + i], d->y[jj], value);
-        d->y[i] = value / d->H[(size_t)i * LDH + i];
+    const int cnt = d->count, lane = threadIdx.x & 31;
+    double value = lane < cnt ? d->g[lane] : 0.;
+    const double diag = lane < cnt ? d->H[(size_t)lane * LDH + lane] : 1.;
+    double above[KR_MAXK];  // the row's entries right of the diagonal
+#pragma unroll
+    for (int i = 0; i < KR_MAXK; ++i) above[i] = i < cnt && lane < i ? d->H[(size_t)i * LDH + lane] : 0.;
+#pragma unroll
+    for (int i = KR_MAXK - 1; i >= 0; --i) {
+        if (i >= cnt) continue;
+        if (lane == i) value = value / diag;
+        const double y = __shfl_sync(0xffffffffu, value, i);
+        if (lane < i) value = rfma(-above[i], y, value);
     }
-    for (int k = 0; k < KR_MAXK; ++k) coef[k] = k < cnt ? d->y[k] : 0.;
+    if (lane < cnt) d->y[lane] = value;
+    coef[lane] = lane < cnt ? value : 0.;
 }
-__global__ void k_gmres_backsolve(GmresDev *d, double *coef) {
-    if (threadIdx.x != 0) return;
-    gmres_backsolve_body(d, coef);
-}
+__global__ void k_gmres_backsolve(GmresDev *d, double *coef) { gmres_backsolve_body(d, coef); }
+static_assert(KR_MAXK == 32, "a lane per basis vector");
 
 // out[i] = sum_{k < *count} V_k[i] c_k with the basis size read on the device.
 __device__ __forceinline__ void lincomb_dyn_body(int bx, int G, const double *__restrict__ V, size_t ldv,

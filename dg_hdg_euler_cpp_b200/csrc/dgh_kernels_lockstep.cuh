@@ -125,15 +125,19 @@ __global__ void __launch_bounds__(KR_THREADS) k_ls_lincomb(const LsMember *t, in
 // ---- GMRES control, one CTA per member ---------------------------------------------------------
 __global__ void k_ls_gmres_init(const LsMember *t) {
     const LsMember &a = t[blockIdx.x];
-    if (threadIdx.x == 0 && ls_on(a, 0)) gmres_init_body(a.gdev, a.red + 2 * KR_MAXK);
+    if (ls_on(a, 0)) gmres_init_body(a.gdev, a.red + 2 * KR_MAXK);
 }
-__global__ void k_ls_gmres_update(const LsMember *t, int j) {
+// (with the reduction of the step's norm before it)
+__global__ void __launch_bounds__(KR_THREADS) k_ls_reduce_update(const LsMember *t, int j) {
     const LsMember &a = t[blockIdx.x];
-    if (threadIdx.x == 0 && ls_on(a, 1)) gmres_update_body(a.gdev, a.red, j);
+    if (!ls_on(a, 1)) return;
+    reduce_body(0, a.partial, a.red_blocks, a.red + 2 * KR_MAXK);
+    __syncthreads();  // (every warp has read the flag, too)
+    if (threadIdx.x < 32) gmres_update_body(a.gdev, a.red, j);
 }
 __global__ void k_ls_gmres_backsolve(const LsMember *t) {
     const LsMember &a = t[blockIdx.x];
-    if (threadIdx.x == 0 && ls_on(a, 0)) gmres_backsolve_body(a.gdev, a.coef);
+    if (ls_on(a, 0)) gmres_backsolve_body(a.gdev, a.coef);
 }
 // flags[i] = member i continues its Arnoldi steps
 __global__ void k_ls_cont(const LsMember *t, int count, int *flags) {
