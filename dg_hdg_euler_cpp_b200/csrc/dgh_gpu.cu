@@ -938,7 +938,7 @@ void dg_apply(dgh_ctx *c, const double *v, double *out) {
     DGH_DISPATCH_N(c->n, {
         using T = Team<N>;
         k_dg_apply<N><<<c->team_blocks(T::CPB), T::THREADS, 0, c->stream>>>(v, c->traces2, c->vol, c->fcache, c->speeds,
-                                                                            out, c->basis_dev, c->g, c->inv_step,
+                                                                            out, c->basis_dev, c->basis, c->g, c->inv_step,
                                                                             c->overint() ? 0 : 1);
         if (c->overint()) {
             k_vol_apply_q<N><<<std::min(c->cells, c->sms * 4), Q_THREADS, 0, c->stream>>>(v, c->volq, out, c->bq, c->g);
@@ -1291,7 +1291,8 @@ void ls_jv_all(dgh_lockstep *L, int src, int dst, int gate) {
         }
         DGH_DISPATCH_N(r.key, {
             k_ls_face_trace<N><<<r.blocks, Team<N>::THREADS, 0, L->stream>>>(L->table, r.first, r.count, src, gate);
-            k_ls_dg_apply<N><<<r.blocks, Team<N>::THREADS, 0, L->stream>>>(L->table, r.first, r.count, src, dst, gate);
+            k_ls_dg_apply<N><<<r.blocks, Team<N>::THREADS, 0, L->stream>>>(L->table, r.first, r.count, src, dst, gate,
+                                                                               L->members[r.first]->basis);
         });
         L->launched(2);
     }
@@ -2621,7 +2622,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
         launch_dg_fused(c, first, count);
         return;
     }
-    if (c->half16()) {  // FP64 left-looking in the workspace, then FP16 slabs with row scales
+    if (c->half16()) {  // FP64 LU in the workspace, then FP16 slabs with row scales
         const int mp = pad8(c->m);
         for (int f = first; f < first + count; f += c->dg_ws_cells) {
             const int cnt = std::min(c->dg_ws_cells, first + count - f);
@@ -2644,7 +2645,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
         return;
     }
     if (c->mixed()) {
-        if (variant == 0) {  // FP64 left-looking in the workspace, FP32 slabs out, chunked
+        if (variant == 0) {  // FP64 LU in the workspace, FP32 slabs out, chunked
             for (int f = first; f < first + count; f += c->dg_ws_cells) {
                 const int cnt = std::min(c->dg_ws_cells, first + count - f);
                 DGH_DISPATCH_N(c->n, {
@@ -3198,13 +3199,13 @@ const double *dgh_gmres_residual(dgh_ctx *c, int op) {
 // ---- Standalone block Jacobi (BlockJacobi, block_jacobi.hpp:7-47) -----------------------------------
 // A pool of `count` dense m x m blocks, factored by one of the device LU kernels and applied as
 // z = A^{-1} x per block.  It runs on a bare context that carries only what the launch helpers
-// read: the stream, the status word, the SM count and the left-looking kernel's scratch.
+// read: the stream, the status word, the SM count and the tensor-pipe kernel's scratch.
 struct dgh_block_jacobi {
     dgh_ctx *c = nullptr;
     int m = 0, count = 0, precision = 0, variant = 0;
     void *pool = nullptr;
     int *perm = nullptr;
-    double *ws = nullptr;  // FP64 workspace of the left-looking kernel in the mixed form
+    double *ws = nullptr;  // FP64 workspace of the tensor-pipe kernel in the mixed form
     bool factored = false;
 };
 

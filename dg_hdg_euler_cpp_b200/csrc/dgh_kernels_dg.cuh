@@ -266,13 +266,14 @@ template <int N>
 __device__ __forceinline__ void dg_apply_body(int bx, const double *__restrict__ d, const double *__restrict__ dtr,
                                               const double *__restrict__ vol, const double *__restrict__ fcache,
                                               const double *__restrict__ speeds, double *__restrict__ out,
-                                              const Basis1D *__restrict__ bp, const Grid &g, double inv_step,
-                                              int volterm) {
-    // the basis tables are indexed per thread: read them through L1 from a device copy rather
-    // than from the kernel's parameter bank, where lane-varying indices serialise
+                                              const Basis1D *__restrict__ bp, const Basis1D &bc, const Grid &g,
+                                              double inv_step, int volterm) {
+    // tables indexed per thread are read through L1 from a device copy (b) rather than from the kernel's
+    // parameter bank (bc), where lane-varying indices serialise
     const Basis1D &b = *bp;
     using T = Team<N>;
-    __shared__ double fx[T::CPB][NVAR * T::P], fy[T::CPB][NVAR * T::P];
+    constexpr int RP = N | 1, VP = N * RP;  // odd row pitch: the lines along x start in different banks
+    __shared__ double fx[T::CPB][NVAR * VP], fy[T::CPB][NVAR * VP];
     __shared__ double ff[T::CPB][NFACES * N * NVAR];
     const int sub = threadIdx.x / T::TPC, lt = threadIdx.x % T::TPC;
     const int cell = bx * T::CPB + sub;
@@ -288,8 +289,8 @@ __device__ __forceinline__ void dg_apply_body(int bx, const double *__restrict__
         normal_action_rn(g.gamma, c[0], c[1], c[2], dd, 1, e);
 #pragma unroll
         for (int v = 0; v < NVAR; ++v) {
-            fx[sub][v * T::P + lt] = a[v];
-            fy[sub][v * T::P + lt] = e[v];
+            fx[sub][v * VP + lt / N * RP + lt % N] = a[v];
+            fy[sub][v * VP + lt / N * RP + lt % N] = e[v];
         }
     }
     if (active)
@@ -316,20 +317,38 @@ __device__ __forceinline__ void dg_apply_body(int bx, const double *__restrict__
                 ff[sub][k * NVAR + v] = rmul(sign, rfma(c[6], al[v], rfma(c[7], ar[v], rmul(pen, rsub(L[v], R[v])))));
         }
     __syncthreads();
+    // the derivatives in place, a thread per line of points (variable, direction): its N values are read once
+    // and multiplied by uniform table entries, which the FMAs take from the parameter bank.  A thread per
+    // point, which reads 2 N values and as many table entries for each variable, was bound by those reads:
+    // 9,216 cells of degree 8 (7, 6) in 46.7 (29.6, 27.6) us, now 35.8 (24.8, 23.6).
+    if (N > 1 && volterm) {
+        if (active)
+            for (int k = lt; k < 2 * NVAR * N; k += T::TPC) {
+                const int v = k / N % NVAR, line = k % N;
+                const bool x = k < NVAR * N;
+                double *p = x ? &fx[sub][v * VP + RP * line] : &fy[sub][v * VP + line];
+                const int step = x ? 1 : RP;
+                double in[N];
+#pragma unroll
+                for (int q = 0; q < N; ++q) in[q] = p[q * step];
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    double s = 0;
+#pragma unroll
+                    for (int q = 0; q < N; ++q) s = rfma(bc.dw[q * N + i], in[q], s);
+                    p[i * step] = s;
+                }
+            }
+        __syncthreads();
+    }
     if (!active || lt >= T::P) return;
     const int ix = lt % N, iy = lt / N;
     const double mass = rmul(rmul(rmul(rmul(.25, g.hx), g.hy), b.w[ix]), b.w[iy]);
     const double sxw = rmul(rmul(.5, g.hy), b.w[iy]), syw = rmul(rmul(.5, g.hx), b.w[ix]);
 #pragma unroll
     for (int v = 0; v < NVAR; ++v) {
-        double wx = 0, wy = 0;
-#pragma unroll
-        for (int q = 0; q < N; ++q) {
-            wx = rfma(b.dw[q * N + ix], fx[sub][v * T::P + q + N * iy], wx);
-            wy = rfma(fy[sub][v * T::P + ix + N * q], b.dw[q * N + iy], wy);
-        }
         double val = rmul(rmul(mass, dd[v]), inv_step);
-        if (N > 1 && volterm) val = rsub(val, rfma(sxw, wx, rmul(syw, wy)));
+        if (N > 1 && volterm) val = rsub(val, rfma(sxw, fx[sub][v * VP + iy * RP + ix], rmul(syw, fy[sub][v * VP + iy * RP + ix])));
         const double lift = rfma(b.eL[ix], ff[sub][(0 * N + iy) * NVAR + v],
                                  rfma(b.eR[ix], ff[sub][(1 * N + iy) * NVAR + v],
                                       rfma(b.eL[iy], ff[sub][(2 * N + ix) * NVAR + v],
@@ -341,8 +360,8 @@ template <int N>
 __global__ void __launch_bounds__(Team<N>::THREADS, 65536 / (Team<N>::THREADS * 72))
 k_dg_apply(const double *__restrict__ d, const double *__restrict__ dtr, const double *__restrict__ vol,
            const double *__restrict__ fcache, const double *__restrict__ speeds, double *__restrict__ out,
-           const Basis1D *__restrict__ bp, Grid g, double inv_step, int volterm = 1) {
-    dg_apply_body<N>(blockIdx.x, d, dtr, vol, fcache, speeds, out, bp, g, inv_step, volterm);
+           const Basis1D *__restrict__ bp, const __grid_constant__ Basis1D bc, Grid g, double inv_step, int volterm = 1) {
+    dg_apply_body<N>(blockIdx.x, d, dtr, vol, fcache, speeds, out, bp, bc, g, inv_step, volterm);
 }
 
 // ---- adjoint J^T w (the transpose of k_dg_apply, same frozen speeds and caches) -------------

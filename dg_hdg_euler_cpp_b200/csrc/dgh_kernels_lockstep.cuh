@@ -210,11 +210,11 @@ __global__ void __launch_bounds__(Team<N>::THREADS) k_ls_face_trace(const LsMemb
 }
 template <int N>
 __global__ void __launch_bounds__(Team<N>::THREADS, 65536 / (Team<N>::THREADS * 72))
-k_ls_dg_apply(const LsMember *t, int first, int count, int src, int dst, int gate) {
+k_ls_dg_apply(const LsMember *t, int first, int count, int src, int dst, int gate, const __grid_constant__ Basis1D bc) {
     const LsMember &a = t[ls_find(t, first, count, blockIdx.x, LS_TEAM)];
     if (!ls_on(a, gate)) return;
     dg_apply_body<N>(blockIdx.x - a.team0, ls_vec(a, src, 0), a.traces, a.vol, a.fcache, a.speeds, ls_vec(a, dst, 0),
-                     a.basis, a.g, a.inv_step, 1);
+                     a.basis, bc, a.g, a.inv_step, 1);
 }
 
 }  // namespace dgh

@@ -101,7 +101,7 @@ def test_fp32_schur_apply_by_degree(k):
 
 
 @pytest.mark.parametrize("restart", [4, 16, 31])
-@pytest.mark.parametrize("nx,ny,k", [(3, 2, 1), (5, 3, 2), (16, 9, 3)])
+@pytest.mark.parametrize("nx,ny,k", [(3, 3, 1), (5, 3, 2), (16, 9, 3)])
 def test_gmres_cycles(nx, ny, k, restart):
     """The reductions, the Hessenberg update and the back substitution at full and partial cycles: the
     returned solution's own residual in the 2-norm, 1e-12 in the solver's weighted norm, whose weights
