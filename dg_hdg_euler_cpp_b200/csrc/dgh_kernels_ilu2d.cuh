@@ -3,7 +3,7 @@
 // 2D front end offers block Jacobi only).  Kernels: the face coupling blocks of DGOperator::block
 // (dg_operator.cpp:22-48, col != row), the level-scheduled forward and backward sweeps of the
 // application, and the block copies and inverse staging of the factorisation.  The batched block products of the
-// factorisation are plain GEMMs (cuBLAS), and the diagonal inverses come from k_lu_left.
+// factorisation are plain GEMMs (cuBLAS), and the diagonal inverses come from k_lu_crout.
 #pragma once
 #include "dgh_kernels_dg.cuh"
 #include "dgh_lu.hpp"

@@ -612,7 +612,7 @@ __global__ void k_round(const double *__restrict__ x, float *__restrict__ y, lon
 
 // Copy of the factored m x m part of each augmented matrix (row length ld) into the slab
 // layout of k_lu_solve (a pool of m x m blocks in TD): one warp per 32-row slab, 16-byte stores.
-// Position i's factor row is source row i, or, with perm, source row perm[i] (the left-looking
+// Position i's factor row is source row i, or, with perm, source row perm[i] (the tensor-pipe
 // LU leaves its factors in original-row order).
 template <typename TS, typename TD>
 __global__ void k_slab_pack(const TS *__restrict__ src, size_t stride, int m, int ld, int count, TD *__restrict__ dst,

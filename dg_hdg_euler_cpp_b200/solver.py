@@ -284,7 +284,7 @@ class Solver:
         self._rc(self.lib.dgh_shape_set(self.h, 0, int(shape)))
 
     def fused_ctas(self, ctas: int):
-        """CTAs per SM of the fused reduced-precision DG factorisation, 1 or 2 (dgh_shape_set)."""
+        """CTAs per SM of the fused DG factorisation: 1, or 2 for all that fit (dgh_shape_set)."""
         self._rc(self.lib.dgh_shape_set(self.h, 1, int(ctas)))
 
     # ---- GMRES
@@ -370,7 +370,7 @@ class Integrator:
 class BlockJacobi:
     """A standalone pool of dense blocks factored on the device (BlockJacobi,
     block_jacobi.hpp:7-47): factor(blocks) with one of the LU kernels, apply(x) = A^{-1} x per
-    block.  variant 0 left-looking FP64 tensor-pipe LU, 1 right-looking blocked LU, 2 one-warp LU
+    block.  variant 0 FP64 tensor-pipe LU, 1 right-looking blocked LU, 2 one-warp LU
     (m <= 64), 3 FP64 LU with FP32 explicit inverses (m <= 64, mixed)."""
 
     def __init__(self, m: int, count: int, precision: str = "fp64", variant: int = 0, device: int = 0):

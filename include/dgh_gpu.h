@@ -203,9 +203,9 @@ int dgh_gmres(dgh_ctx *ctx, int op, const double *rhs, double *x, int limit, dou
 /* Per-degree autotuner (no counterpart in the reference).  With dgh_config.autotune set, the
  * first DG block-Jacobi refresh and the first HDG condensation of a context time their
  * factorisation variants on a sample of the context's own cells and keep the faster one; the
- * choice is cached per (degree, precision) for the process.  Variants: DG blocks 0 = left-looking
- * FP64 LU on the tensor pipe (FP32 slabs in the mixed form), 1 = right-looking LU (FP32 in the
- * mixed form); condensation 0 = left-looking LU with the fused right-hand-side solve,
+ * choice is cached per (degree, precision) for the process.  Variants: DG blocks 0 = FP64
+ * LU on the tensor pipe (FP32 slabs in the mixed form), 1 = right-looking LU (FP32 in the
+ * mixed form); condensation 0 = tensor-pipe LU with the fused right-hand-side solve,
  * 1 = right-looking LU then the tensor-pipe back substitution.  All variants compute the same
  * factors up to rounding.  out[0..1] = the DG and condensation variants in use, -1 where the
  * context has not factored yet; out[2..5] = the last tuning times in ms (DG 0, DG 1, HDG 0,
@@ -215,8 +215,8 @@ int dgh_autotune_report(const dgh_ctx *ctx, double out[6]);
  * reference).  DGH_SHAPE_SOLVE_GRID: the grid of the 2D DG block-Jacobi solves, 0 = every
  * resident CTA slot, 1 = the fewest CTAs with the same number of rounds of blocks per warp (equal
  * shares); timed at the first DG refresh on the context's own factors, cached per (degree,
- * precision, cell count); default 0.  DGH_SHAPE_FUSED_CTAS: CTAs per SM of the fused reduced-
- * precision DG factorisation, 1 (each CTA's FP64 slot fits L2) or 2 (twice the warps); timed at
+ * precision, cell count); default 0.  DGH_SHAPE_FUSED_CTAS: CTAs per SM of the fused
+ * DG factorisation, 1 (each CTA's FP64 slot fits L2) or 2 (every CTA that is resident); timed at
  * the first DG refresh on a sample of the cells, cached per (degree, precision); default 2.
  * dgh_shape_set fixes a shape instead; every shape computes the same bits.
  * dgh_autotune_shapes: out[0] = the solve grid shape in use (-1 before the first DG refresh),
@@ -275,7 +275,7 @@ int dgh_integrator_set_limits(dgh_integrator *it, int hdg_attempts, int line_sea
  * (the first largest |a| wins ties, as LAPACK getrf / Eigen PartialPivLU) by one device LU kernel,
  * then applied as z = A^{-1} x block by block (block_jacobi.hpp:24-39).  blocks, x and z are device
  * pointers; blocks are row-major FP64 and are copied (the caller keeps them).  variant: 0 the
- * left-looking FP64 LU on the tensor pipe, 1 the right-looking blocked LU, 2 the one-warp LU for
+ * FP64 LU on the tensor pipe, 1 the right-looking blocked LU, 2 the one-warp LU for
  * narrow blocks (m <= 64), 3 FP64 LU with explicit inverses stored in FP32 (m <= 64, mixed only).
  * precision DGH_PRECISION_MIXED stores the factors in FP32 (variant 1 and 2 factor in FP32).  A
  * block with a zero, subnormal or non-finite pivot fails with DGH_ERR_SINGULAR ("Singular block
