@@ -122,6 +122,7 @@ struct dgh_ctx {
     // DG block Jacobi pool (precision per cfg.precision)
     void *dg_pool = nullptr;
     int *dg_perm = nullptr;
+    unsigned char *dg_kept = nullptr;  // FP64 slabs: a byte per diagonal square (k_slab_invert)
     // HDG condensation
     double *S = nullptr, *X = nullptr, *Y = nullptr, *cy = nullptr, *hrhs = nullptr;
     double *aug = nullptr;
@@ -130,6 +131,7 @@ struct dgh_ctx {
     size_t aug_bytes = 0;
     void *face_pool = nullptr;
     int *face_perm = nullptr;
+    unsigned char *face_kept = nullptr;
     bool face_inverse = false;  // mixed 2D: face_pool holds FP32 explicit inverses
     // FP32 condensation (dgh_config.condense32, 2D): the cells' LU factors of A in FP32 slabs
     // with their permutations, the Schur blocks in FP32, the FP32 view of the condensation
@@ -508,16 +510,16 @@ void interior_cells(const dgh_ctx *c, int &first, int &count) {
     count = c->slabbed() ? c->g.nx * c->slab.rows : c->cells;
 }
 
-// Panel width 32; U12 tile width 32 for FP64 (two CTAs per SM fit in shared memory at m = 324)
-// and 64 for FP32.
-// The FP64 slabs' diagonal squares inverted in place: the last step of every factorisation that leaves FP64
-// slabs.
-void launch_slab_invert(dgh_ctx *c, double *pool, int m, int count) {
-    const long long squares = (long long)count * ((m + 31) / 32);
+// The FP64 slabs' diagonal squares inverted in place, but for the kept ones: the last step of every
+// factorisation that leaves FP64 slabs.
+void launch_slab_invert(dgh_ctx *c, double *pool, int m, int count, unsigned char *kept) {
+    const long long squares = (long long)count * slab_count(m);
     k_slab_invert<<<(unsigned)((squares + SQUARE_WARPS - 1) / SQUARE_WARPS), 32 * SQUARE_WARPS, 0, c->stream>>>(
-        pool, (size_t)m * m, m, count);
+        pool, (size_t)m * m, m, count, kept);
     c->launched();
 }
+// Panel width 32; U12 tile width 32 for FP64 (two CTAs per SM fit in shared memory at m = 324)
+// and 64 for FP32.
 constexpr int LU_NB = 32;
 template <typename TF> constexpr int lu_tc() { return sizeof(TF) == 8 ? 32 : 64; }
 template <typename TF> void setup_lu_attrs(size_t smem) {
@@ -525,7 +527,7 @@ template <typename TF> void setup_lu_attrs(size_t smem) {
 }
 template <typename TF>
 void launch_lu(dgh_ctx *c, TF *pool, size_t stride, int m, int ld, int count, int *perm, int bit, bool slab_out,
-               bool lfix = false) {
+               bool lfix = false, unsigned char *kept = nullptr) {
     constexpr int TC = lu_tc<TF>();
     const size_t smem = lu_smem_bytes<TF, LU_NB, TC>(m);
     setup_lu_attrs<TF>(smem);
@@ -536,13 +538,14 @@ void launch_lu(dgh_ctx *c, TF *pool, size_t stride, int m, int ld, int count, in
                                                                slab_out ? 3 : lfix ? 2 : 0);
     c->launched();
     if constexpr (sizeof(TF) == 8)
-        if (slab_out) launch_slab_invert(c, pool, m, count);
+        if (slab_out) launch_slab_invert(c, pool, m, count, kept);
 }
 // The FP64 LU on the tensor pipe (dgh_kernels_lu2.cuh) of m x m blocks, in place or to FP32 slabs.
-void launch_lu_pool(dgh_ctx *c, double *pool, int m, int count, int *perm, int bit, bool slab_out, float *out32 = nullptr) {
+void launch_lu_pool(dgh_ctx *c, double *pool, int m, int count, int *perm, int bit, unsigned char *kept, float *out32 = nullptr) {
+    const bool slab_out = kept != nullptr;
     lu_pool({c->stream, c->sms, c->status, bit}, pool, m, count, perm, slab_out, out32);
     c->launched();
-    if (slab_out && !out32) launch_slab_invert(c, pool, m, count);
+    if (slab_out) launch_slab_invert(c, pool, m, count, kept);
 }
 // The same with t + 1 augmented columns: X | y = A^{-1} [B | r], to x and y.
 void launch_lu_augmented(dgh_ctx *c, double *aug, int m, int t, int count, int *perm, int bit, double *x, double *y) {
@@ -575,12 +578,12 @@ void launch_dg_fused(dgh_ctx *c, int first, int count) {
     }
     lu_fused({c->stream, c->sms, c->status, ST_SINGULAR}, c->n, fu, grid, count, c->dg_perm + (size_t)first * c->m, out32);
     c->launched();
-    if (fu.out64) launch_slab_invert(c, fu.out64, c->m, count);
+    if (fu.out64) launch_slab_invert(c, fu.out64, c->m, count, c->dg_kept + (size_t)first * slab_count(c->m));
 }
 
 // Narrow blocks (m <= 64): one warp per block in shared memory.
 template <typename TF>
-void launch_lu_narrow(dgh_ctx *c, TF *pool, int m, int count, int *perm, int bit) {
+void launch_lu_narrow(dgh_ctx *c, TF *pool, int m, int count, int *perm, int bit, unsigned char *kept = nullptr) {
     need(m <= 64 && m % 4 == 0, "block width unsupported by the narrow LU");
     const size_t smem = lu_narrow_smem_bytes<TF>(m);
     allow_dynamic_smem((const void *)k_lu_narrow<TF>, smem);
@@ -590,7 +593,7 @@ void launch_lu_narrow(dgh_ctx *c, TF *pool, int m, int count, int *perm, int bit
     const int grid = std::min((count + wpc - 1) / wpc, c->sms * std::max(1, resident));
     k_lu_narrow<TF><<<grid, NARROW_THREADS, smem, c->stream>>>(pool, m, count, perm, c->status, bit);
     c->launched();
-    if constexpr (sizeof(TF) == 8) launch_slab_invert(c, pool, m, count);
+    if constexpr (sizeof(TF) == 8) launch_slab_invert(c, pool, m, count, kept);
 }
 // Grid of a one-warp-per-block solve over `count` blocks with `wpc` warps per CTA and `resident`
 // CTAs per SM.  Shape 0 fills every resident CTA slot, so the last round of blocks runs on the
@@ -608,24 +611,24 @@ int solve_grid(const dgh_ctx *c, long long count, int wpc, int resident, int sha
 // One warp per block (dgh_kernels_solve.cuh).
 template <typename TF>
 void launch_solve(dgh_ctx *c, const TF *pool, const int *perm, size_t stride, int m, int count, const double *x,
-                  double *z, int shape = 0, const float *scale = nullptr) {
+                  double *z, int shape = 0, const typename SolveType<TF>::Aux *aux = nullptr) {
     const size_t smem = SOLVE_WARPS * solve_warp_bytes<TF>(m);
     allow_dynamic_smem((const void *)k_lu_solve<TF>, smem);
     int resident = 0;
     ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_lu_solve<TF>, SOLVE_THREADS, smem), "occupancy");
     const int grid = solve_grid(c, count, SOLVE_WARPS, resident, shape);
-    k_lu_solve<TF><<<grid, SOLVE_THREADS, smem, c->stream>>>(pool, scale, perm, stride, m, count, x, z);
+    k_lu_solve<TF><<<grid, SOLVE_THREADS, smem, c->stream>>>(pool, aux, perm, stride, m, count, x, z);
     c->launched();
 }
 template <typename TF>
 void launch_solve_t(dgh_ctx *c, const TF *pool, const int *perm, size_t stride, int m, int count, const double *x,
-                    double *z) {
+                    double *z, const typename SolveType<TF>::Aux *aux = nullptr) {
     const size_t smem = SOLVE_WARPS * solve_warp_bytes<TF, true>(m);
     allow_dynamic_smem((const void *)k_lu_solve_t<TF>, smem);
     int resident = 0;
     ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_lu_solve_t<TF>, SOLVE_THREADS, smem), "occupancy");
     const int grid = solve_grid(c, count, SOLVE_WARPS, resident, 0);
-    k_lu_solve_t<TF><<<grid, SOLVE_THREADS, smem, c->stream>>>(pool, perm, stride, m, count, x, z);
+    k_lu_solve_t<TF><<<grid, SOLVE_THREADS, smem, c->stream>>>(pool, aux, perm, stride, m, count, x, z);
     c->launched();
 }
 
@@ -866,7 +869,7 @@ void dg_block_solve(dgh_ctx *c, int shape, const double *x, double *z) {
         launch_solve<__half>(c, (const __half *)c->dg_pool, c->dg_perm, (size_t)c->m * pad8(c->m), c->m, c->cells, x, z, shape,
                              c->dg_scale);
     else if (c->mixed()) launch_solve<float>(c, (const float *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z, shape);
-    else launch_solve<double>(c, (const double *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z, shape);
+    else launch_solve<double>(c, (const double *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z, shape, c->dg_kept);
 }
 void precond_apply(dgh_ctx *c, int op, const double *x, double *z) {
     Timed tm(c, DGH_TIMER_PRECOND);
@@ -897,7 +900,7 @@ void precond_apply(dgh_ctx *c, int op, const double *x, double *z) {
         need(!c->half16(), "The transposed solve needs FP64 or FP32 factors");
         need(!c->ilu2d(), "The transposed block ILU(0) is not built");
         if (c->mixed()) launch_solve_t<float>(c, (const float *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z);
-        else launch_solve_t<double>(c, (const double *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z);
+        else launch_solve_t<double>(c, (const double *)c->dg_pool, c->dg_perm, stride, c->m, c->cells, x, z, c->dg_kept);
         return;
     }
     if (op == DGH_OP_DG && c->ilu2d()) {
@@ -919,7 +922,7 @@ void precond_apply(dgh_ctx *c, int op, const double *x, double *z) {
             c->launched();
         } else if (c->mixed())
             launch_solve<float>(c, (const float *)c->face_pool, c->face_perm, stride, c->fw, c->faces, x, z);
-        else launch_solve<double>(c, (const double *)c->face_pool, c->face_perm, stride, c->fw, c->faces, x, z);
+        else launch_solve<double>(c, (const double *)c->face_pool, c->face_perm, stride, c->fw, c->faces, x, z, 0, c->face_kept);
     }
 }
 
@@ -1328,6 +1331,7 @@ void ls_plan_face_precond(dgh_lockstep *L) {
         L->host[i].solve0 = lr.blocks;
         L->host[i].pool = c->face_pool;
         L->host[i].perm = c->face_perm;
+        L->host[i].kept = c->face_kept;
         constexpr int inv_wpc = INV_APPLY_THREADS / 32;
         lr.blocks += key == 4 ? (c->faces + inv_wpc - 1) / inv_wpc : ls_solve_blocks(c, c->faces);
         ++lr.count;
@@ -2075,6 +2079,7 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
                 c->dg_scale = c->alloc<float>((size_t)c->cells * c->m);
             } else {
                 c->dg_pool = c->alloc<char>((size_t)c->cells * c->m * c->m * tsz);
+                if (!c->mixed()) c->dg_kept = c->alloc<unsigned char>((size_t)c->cells * slab_count(c->m));
             }
             c->dg_perm = c->alloc<int>((size_t)c->cells * c->m);
         }
@@ -2101,6 +2106,7 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
             c->aug_perm = c->alloc<int>((size_t)c->aug_cells * c->m);
             c->face_pool = c->alloc<char>((size_t)c->faces * c->fw * c->fw * tsz);
             c->face_perm = c->alloc<int>((size_t)c->faces * c->fw);
+            if (!c->mixed()) c->face_kept = c->alloc<unsigned char>((size_t)c->faces * slab_count(c->fw));
         }
         const long long vn = std::max(c->has_dg() ? c->N : 0LL, c->has_hdg() ? c->NT : 0LL);
         c->vld = ((vn + 31) / 32) * 32;
@@ -2636,7 +2642,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
                 }
             });
             c->launched();
-            launch_lu_pool(c, c->dg_ws, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR, false);
+            launch_lu_pool(c, c->dg_ws, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR, nullptr);
             const long long warps = (long long)cnt * ((c->m + 31) / 32);
             k_pack_half<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, c->stream>>>(
                 c->dg_ws, c->m, cnt, (__half *)c->dg_pool + (size_t)f * c->m * mp, c->dg_scale + (size_t)f * c->m);
@@ -2658,7 +2664,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
                     }
                 });
                 c->launched();
-                launch_lu_pool(c, c->dg_ws, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR, false,
+                launch_lu_pool(c, c->dg_ws, c->m, cnt, c->dg_perm + (size_t)f * c->m, ST_SINGULAR, nullptr,
                                (float *)c->dg_pool + (size_t)f * stride);
             }
         } else {  // FP32 right-looking in place
@@ -2677,6 +2683,7 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
         }
     } else {
         double *pool = (double *)c->dg_pool + (size_t)first * stride;
+        unsigned char *kept = c->dg_kept + (size_t)first * slab_count(c->m);
         DGH_DISPATCH_N(c->n, {
             k_dg_assemble<N, double><<<grid, 256, 0, c->stream>>>(pool, c->vol, c->fcache, c->speeds, c->basis, c->g,
                                                                   c->inv_step, first, count, c->overint() ? 0 : 1);
@@ -2688,9 +2695,10 @@ void dg_factor(dgh_ctx *c, int variant, int first, int count) {
         });
         c->launched();
         if (variant == 0)
-            launch_lu_pool(c, pool, c->m, count, c->dg_perm + (size_t)first * c->m, ST_SINGULAR, true);
+            launch_lu_pool(c, pool, c->m, count, c->dg_perm + (size_t)first * c->m, ST_SINGULAR, kept);
         else
-            launch_lu<double>(c, pool, stride, c->m, c->m, count, c->dg_perm + (size_t)first * c->m, ST_SINGULAR, true);
+            launch_lu<double>(c, pool, stride, c->m, c->m, count, c->dg_perm + (size_t)first * c->m, ST_SINGULAR, true,
+                              false, kept);
     }
 }
 // Condensation of cells [first, first + count) (count <= aug_cells): [A | B | r], LU + solve
@@ -2978,7 +2986,7 @@ int dgh_block_jacobi_refresh(dgh_ctx *c, int op) {
                 launch_lu_narrow<float>(c, (float *)c->face_pool, c->fw, c->faces, c->face_perm, ST_SINGULAR);
             } else {
                 face_blocks<double>(c, (double *)c->face_pool);
-                launch_lu_narrow<double>(c, (double *)c->face_pool, c->fw, c->faces, c->face_perm, ST_SINGULAR);
+                launch_lu_narrow<double>(c, (double *)c->face_pool, c->fw, c->faces, c->face_perm, ST_SINGULAR, c->face_kept);
             }
             c->check_status();
             c->face_factored = true;
@@ -3205,6 +3213,7 @@ struct dgh_block_jacobi {
     int m = 0, count = 0, precision = 0, variant = 0;
     void *pool = nullptr;
     int *perm = nullptr;
+    unsigned char *kept = nullptr;  // FP64: a byte per diagonal square (k_slab_invert)
     double *ws = nullptr;  // FP64 workspace of the tensor-pipe kernel in the mixed form
     bool factored = false;
 };
@@ -3245,6 +3254,7 @@ int dgh_block_jacobi_create(int m, int count, int precision, int variant, int de
         const size_t tsz = precision == DGH_PRECISION_MIXED ? sizeof(float) : sizeof(double);
         bj->pool = c->alloc<char>((size_t)count * m * m * tsz);
         bj->perm = c->alloc<int>((size_t)count * m);
+        if (precision == DGH_PRECISION_FP64) bj->kept = c->alloc<unsigned char>((size_t)count * slab_count(m));
         if (precision == DGH_PRECISION_MIXED && (variant == 0 || variant == 3))
             bj->ws = c->alloc<double>((size_t)count * m * m);
         c->sync();
@@ -3280,15 +3290,15 @@ int dgh_block_jacobi_factor(dgh_block_jacobi *bj, const double *blocks) {
         if (bj->precision == DGH_PRECISION_FP64) {
             double *pool = (double *)bj->pool;
             ck(cudaMemcpyAsync(pool, blocks, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy blocks");
-            if (bj->variant == 0) launch_lu_pool(c, pool, m, count, bj->perm, ST_SINGULAR, true);
-            else if (bj->variant == 1) launch_lu<double>(c, pool, stride, m, m, count, bj->perm, ST_SINGULAR, true);
-            else launch_lu_narrow<double>(c, pool, m, count, bj->perm, ST_SINGULAR);
+            if (bj->variant == 0) launch_lu_pool(c, pool, m, count, bj->perm, ST_SINGULAR, bj->kept);
+            else if (bj->variant == 1) launch_lu<double>(c, pool, stride, m, m, count, bj->perm, ST_SINGULAR, true, false, bj->kept);
+            else launch_lu_narrow<double>(c, pool, m, count, bj->perm, ST_SINGULAR, bj->kept);
         } else {
             float *pool = (float *)bj->pool;
             if (bj->variant == 0 || bj->variant == 3) {
                 ck(cudaMemcpyAsync(bj->ws, blocks, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy blocks");
                 if (bj->variant == 0) {
-                    launch_lu_pool(c, bj->ws, m, count, bj->perm, ST_SINGULAR, false, pool);
+                    launch_lu_pool(c, bj->ws, m, count, bj->perm, ST_SINGULAR, nullptr, pool);
                 } else {
                     const size_t smem = inv_narrow_smem_bytes(m);
                     allow_dynamic_smem((const void *)k_inv_narrow, smem);
@@ -3328,7 +3338,7 @@ int dgh_block_jacobi_apply(dgh_block_jacobi *bj, const double *x, double *z) {
         } else if (bj->precision == DGH_PRECISION_MIXED) {
             launch_solve<float>(c, (const float *)bj->pool, bj->perm, stride, m, count, x, z);
         } else {
-            launch_solve<double>(c, (const double *)bj->pool, bj->perm, stride, m, count, x, z);
+            launch_solve<double>(c, (const double *)bj->pool, bj->perm, stride, m, count, x, z, 0, bj->kept);
         }
         c->sync();
     });
@@ -3453,6 +3463,7 @@ int dgh_lockstep_create_op(dgh_ctx *const *members, int count, int op, dgh_locks
                 t.pool = c->dg_pool;
                 t.scale = c->dg_scale;
                 t.perm = c->dg_perm;
+                t.kept = c->dg_kept;
                 t.stride = (size_t)c->m * (c->half16() ? pad8(c->m) : c->m);
                 t.m = c->m;
                 t.cells = c->cells;

@@ -30,6 +30,7 @@ struct LsMember {
     // block-Jacobi factors (FP64 / FP32 slabs, or FP16 slabs with row scales)
     const void *pool;
     const float *scale;
+    const unsigned char *kept;
     const int *perm;
     size_t stride;
     int m, cells;
@@ -173,7 +174,10 @@ k_ls_solve(const LsMember *t, int first, int count, int src, int dst, int j, int
     const LsMember &a = t[i];
     if (!ls_on(a, gate)) return;
     const int blocks = (i + 1 < first + count ? t[i + 1].solve0 : gridDim.x) - a.solve0;
-    lu_solve_body<T>(blockIdx.x - a.solve0, blocks, (const T *)a.pool, a.scale, a.perm, a.stride, a.m, a.cells,
+    const typename SolveType<T>::Aux *aux;
+    if constexpr (sizeof(T) == 8) aux = a.kept;
+    else aux = a.scale;
+    lu_solve_body<T>(blockIdx.x - a.solve0, blocks, (const T *)a.pool, aux, a.perm, a.stride, a.m, a.cells,
                      ls_vec(a, src, j), ls_vec(a, dst, j));
 }
 

@@ -10,9 +10,11 @@
 //    instructions (with chunks cut by size and not by columns FP16 was bound by its instructions: 3.44 ms
 //    in the last case below);
 //  - the 32 x 32 diagonal triangles of the FP64 factors are stored inverted (k_slab_invert), so a triangle
-//    is one more product instead of 32 dependent steps of a shuffle, an FMA and, going up, a division.
-//    Solutions are as accurate (cells of degree 2 to 8 against 64-bit solves: 3.4e-15 to 6.4e-14 with the
-//    inverses, 3.1e-15 to 6.4e-14 without).  The FP32 and FP16 factors keep their triangles, since inverses
+//    is one more product instead of 32 dependent steps of a shuffle, an FMA and, going up, a division.  A
+//    product's residual grows with the triangle's condition, substitution's does not, so a triangle above
+//    INVERT_BOUND stays as it is, marked in a byte per square, and is solved by substitution.  On cell blocks
+//    of degree 2 to 8 (condition at most 70) solutions are 3.4e-15 to 6.4e-14 from 64-bit solves with the
+//    inverses, 3.1e-15 to 6.4e-14 without.  The FP32 and FP16 factors keep their triangles, since inverses
 //    rounded to FP32 did lose accuracy, and solve them four columns to a shuffle, with the
 //    reciprocals of the diagonal taken beforehand;
 //  - a last slab of 4, 8 or 16 rows gives a row's column groups to 8, 4 or 2 lanes.
@@ -32,13 +34,16 @@ constexpr int SOLVE_WARPS = 4, SOLVE_THREADS = 32 * SOLVE_WARPS;
 
 // Arithmetic type, elements per 16 bytes, columns per chunk, chunks in a warp's ring and row length of a
 // block's slabs, by storage type.
+// Aux: per block, the kept squares of FP64 factors (KEPT_L, KEPT_U) or the row scales of FP16 factors.
 template <typename T> struct SolveType {
     using A = T;
+    using Aux = typename std::conditional<sizeof(T) == 8, unsigned char, float>::type;
     static constexpr int W = SlabVec<T>::W, CW = sizeof(T) == 8 ? 16 : 32, STAGES = 2;
     __host__ __device__ static constexpr int row(int m) { return m; }
 };
 template <> struct SolveType<__half> {
     using A = float;
+    using Aux = float;
     static constexpr int W = H_W, CW = 32, STAGES = 3;
     __host__ __device__ static constexpr int row(int m) { return pad8(m); }
 };
@@ -356,11 +361,20 @@ __device__ __forceinline__ float slab_triangle_t(const uint4 *base, int lane, in
     return triangle<true, false, true>(t, lane, nt, square_at(base, nt, col, col, tag), own, four);
 }
 
-// z = A^{-1} b.  T: the factors' storage; FP16 factors carry row scales (scale: the reciprocal of each U
-// row's largest entry).  The body takes its block index bx and block count G explicitly (the batched
+// Squares of FP64 factors whose triangle is kept (k_slab_invert): a byte per square, slab by slab.
+constexpr unsigned char KEPT_L = 1, KEPT_U = 2;
+// Lane s's byte of block blk, loaded beside the block's vector; ballots make it bits per slab.
+template <typename T> __device__ __forceinline__ int kept_square(const typename SolveType<T>::Aux *aux, int blk, int slabs) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (sizeof(T) == 8) return lane < slabs ? aux[(size_t)blk * slabs + lane] : 0;
+    return 0;
+}
+
+// z = A^{-1} b.  T: the factors' storage; FP16 factors carry row scales (aux: the reciprocal of each U
+// row's largest entry), FP64 factors their kept squares.  The body takes its block index bx and block count G explicitly (the batched
 // solve of a lockstep batch runs it over each member's blocks).
 template <typename T, class Stream>
-__device__ __forceinline__ void lu_solve_blocks(int bx, int G, const T *__restrict__ pool, const float *__restrict__ scale,
+__device__ __forceinline__ void lu_solve_blocks(int bx, int G, const T *__restrict__ pool, const typename SolveType<T>::Aux *__restrict__ aux,
                                               const int *__restrict__ perm, size_t stride, int m, int count,
                                               const double *__restrict__ rhs, double *__restrict__ z) {
     using S = SolveType<T>;
@@ -379,7 +393,13 @@ __device__ __forceinline__ void lu_solve_blocks(int bx, int G, const T *__restri
         in.block(blk);
         const int *pm = perm + (size_t)blk * m;
         const double *b = rhs + (size_t)blk * m;
+        const int kept = kept_square<T>(aux, blk, slabs);
         for (int i = lane; i < ml; i += 32) y[i] = i < m ? (A)b[pm[i]] : A(0);
+        unsigned kept_l = 0, kept_u = 0;
+        if constexpr (sizeof(T) == 8) {
+            kept_l = __ballot_sync(0xffffffffu, kept & KEPT_L);
+            kept_u = __ballot_sync(0xffffffffu, kept & KEPT_U);
+        }
         __syncwarp();
         // sweep 0: forward, L y = P b (columns left of the slab); sweep 1: backward, U z = y (right of it)
         for (int dir = 0; dir < 2; ++dir)
@@ -426,9 +446,26 @@ __device__ __forceinline__ void lu_solve_blocks(int bx, int G, const T *__restri
                     __syncwarp();
                     float t = 0.f;
                     if (lane < nt)
-                        t = sizeof(T) == 2 && dir == 1 ? fmaf(y[r0 + lane], scale[(size_t)blk * m + r0 + lane], -off)
+                        t = sizeof(T) == 2 && dir == 1 ? fmaf(y[r0 + lane], aux[(size_t)blk * m + r0 + lane], -off)
                                                        : y[r0 + lane] - off;
                     t = slab_triangle<T>(square, lane, nt, dir, t);
+                    if (lane < nt) y[r0 + lane] = t;
+                    __syncwarp();
+                } else if ((dir == 0 ? kept_l : kept_u) >> s & 1) {  // substitution, a column at a time
+                    A t = lane < nt ? y[r0 + lane] - off : A(0);
+                    for (int i = 0; i < d1 - d0; ++i) {
+                        const T *e = reinterpret_cast<const T *>(ring + in.next()) + W * lane;
+                        __syncwarp();
+                        const int c0 = CW * (dir == 0 ? i : d1 - d0 - 1 - i), nc = min(CW, nt - c0);
+                        for (int k = 0; k < nc; ++k) {
+                            const int j = dir == 0 ? k : nc - 1 - k, c = c0 + j;
+                            const T a = lane < nt && (dir == 0 ? lane > c : lane <= c) ? e[j / W * nt * W + j % W] : T(1);
+                            if (dir == 1 && lane == c) t = t / a;
+                            const A yc = __shfl_sync(0xffffffffu, t, c);
+                            if (lane < nt && (dir == 0 ? lane > c : lane < c)) t = fma(-a, yc, t);
+                        }
+                        __syncwarp();
+                    }
                     if (lane < nt) y[r0 + lane] = t;
                     __syncwarp();
                 } else {  // the inverted triangle: the slab's right-hand side to y, then one more product
@@ -462,17 +499,17 @@ __device__ __forceinline__ void lu_solve_blocks(int bx, int G, const T *__restri
     }
 }
 template <typename T>
-__device__ __forceinline__ void lu_solve_body(int bx, int G, const T *__restrict__ pool, const float *__restrict__ scale,
+__device__ __forceinline__ void lu_solve_body(int bx, int G, const T *__restrict__ pool, const typename SolveType<T>::Aux *__restrict__ aux,
                                               const int *__restrict__ perm, size_t stride, int m, int count,
                                               const double *__restrict__ rhs, double *__restrict__ z) {
-    if (solve_whole<T>(m)) lu_solve_blocks<T, SlabWhole<T, false>>(bx, G, pool, scale, perm, stride, m, count, rhs, z);
-    else lu_solve_blocks<T, SlabStream<T, false>>(bx, G, pool, scale, perm, stride, m, count, rhs, z);
+    if (solve_whole<T>(m)) lu_solve_blocks<T, SlabWhole<T, false>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
+    else lu_solve_blocks<T, SlabStream<T, false>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
 }
 template <typename T>
 __global__ void __launch_bounds__(SOLVE_THREADS, SOLVE_CTAS<T>)
-k_lu_solve(const T *__restrict__ pool, const float *__restrict__ scale, const int *__restrict__ perm, size_t stride, int m,
+k_lu_solve(const T *__restrict__ pool, const typename SolveType<T>::Aux *__restrict__ aux, const int *__restrict__ perm, size_t stride, int m,
            int count, const double *__restrict__ rhs, double *__restrict__ z) {
-    lu_solve_body<T>(blockIdx.x, gridDim.x, pool, scale, perm, stride, m, count, rhs, z);
+    lu_solve_body<T>(blockIdx.x, gridDim.x, pool, aux, perm, stride, m, count, rhs, z);
 }
 
 // z = A^{-T} b with the same factors (A = P^T L U, so A^{-T} b = P^T L^{-T} U^{-T} b): a forward solve with
@@ -481,8 +518,9 @@ k_lu_solve(const T *__restrict__ pool, const float *__restrict__ scale, const in
 // A lane owns a column of the chunk and walks its rows; the lanes start at different rows, so that a
 // step's elements (and the unknowns they multiply) lie in different banks.
 template <typename T, class Stream>
-__device__ __forceinline__ void lu_solve_t_blocks(const T *__restrict__ pool, const int *__restrict__ perm, size_t stride, int m,
-                                                  int count, const double *__restrict__ rhs, double *__restrict__ z) {
+__device__ __forceinline__ void lu_solve_t_blocks(const T *__restrict__ pool, const typename SolveType<T>::Aux *__restrict__ aux,
+                                                  const int *__restrict__ perm, size_t stride, int m, int count,
+                                                  const double *__restrict__ rhs, double *__restrict__ z) {
     using S = SolveType<T>;
     constexpr int W = S::W, CW = S::CW, D = 32 / CW, PARTS = 32 / CW;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -499,6 +537,12 @@ __device__ __forceinline__ void lu_solve_t_blocks(const T *__restrict__ pool, co
         const int *pm = perm + (size_t)blk * m;
         const double *b = rhs + (size_t)blk * m;
         for (int i = lane; i < m; i += 32) y[i] = (T)b[i];
+        unsigned kept_l = 0, kept_u = 0;
+        if constexpr (sizeof(T) == 8) {
+            const int kept = kept_square<T>(aux, blk, slabs);
+            kept_l = __ballot_sync(0xffffffffu, kept & KEPT_L);
+            kept_u = __ballot_sync(0xffffffffu, kept & KEPT_U);
+        }
         for (int dir = 0; dir < 2; ++dir)
             for (int si = 0; si < slabs; ++si) {
                 const int s = dir == 0 ? si : slabs - 1 - si, r0 = 32 * s, nt = min(32, m - r0), span = nt / PARTS;
@@ -536,6 +580,26 @@ __device__ __forceinline__ void lu_solve_t_blocks(const T *__restrict__ pool, co
                         const float t = slab_triangle_t(reinterpret_cast<const uint4 *>(chunk), lane, nt, dir,
                                                         lane < nt ? (float)y[r0 + lane] : 0.f);
                         if (lane < nt) y[r0 + lane] = t;
+                    } else if ((dir == 0 ? kept_u : kept_l) >> s & 1) {
+                        // the chunk's columns c0..c0 + nc - 1: the rows of known unknowns, halved between the
+                        // lanes of a column, then the triangle, whose pivots are the chunk's own unknowns
+                        const int c0 = CW * jc - r0, nc = min(CW, nt - c0);
+                        const T *a = reinterpret_cast<const T *>(chunk) + q * nt * W + col % W;  // row r: a[r W]
+                        const int lo = dir == 0 ? 0 : c0 + nc, hi = dir == 0 ? c0 : nt;
+                        if (j < m)
+                            for (int r = lo + part; r < hi; r += PARTS) s0 = fma(a[r * W], y[r0 + r], s0);
+#pragma unroll
+                        for (int o = CW; o < 32; o <<= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                        T t = j < m ? y[j] - s0 : T(0);
+                        for (int k = 0; k < nc; ++k) {
+                            const int r = dir == 0 ? k : nc - 1 - k;
+                            const T e = j < m && (dir == 0 ? col >= r : col < r) ? a[(c0 + r) * W] : T(1);
+                            if (dir == 0 && col == r) t = t / e;
+                            const T xr = __shfl_sync(0xffffffffu, t, r);
+                            if (j < m && (dir == 0 ? col > r : col < r)) t = fma(-e, xr, t);
+                        }
+                        __syncwarp();
+                        if (part == 0 && j < m) y[j] = t;
                     } else {  // its inverse
                         const int cc = j - r0 - part * span;  // the diagonal's row, counted from yr
                         if (j < m) {
@@ -564,19 +628,34 @@ __device__ __forceinline__ void lu_solve_t_blocks(const T *__restrict__ pool, co
 
 template <typename T>
 __global__ void __launch_bounds__(SOLVE_THREADS, 4)
-k_lu_solve_t(const T *__restrict__ pool, const int *__restrict__ perm, size_t stride, int m, int count,
-             const double *__restrict__ rhs, double *__restrict__ z) {
-    if (solve_whole<T>(m)) lu_solve_t_blocks<T, SlabWhole<T, true>>(pool, perm, stride, m, count, rhs, z);
-    else lu_solve_t_blocks<T, SlabStream<T, true>>(pool, perm, stride, m, count, rhs, z);
+k_lu_solve_t(const T *__restrict__ pool, const typename SolveType<T>::Aux *__restrict__ aux, const int *__restrict__ perm,
+             size_t stride, int m, int count, const double *__restrict__ rhs, double *__restrict__ z) {
+    if (solve_whole<T>(m)) lu_solve_t_blocks<T, SlabWhole<T, true>>(pool, aux, perm, stride, m, count, rhs, z);
+    else lu_solve_t_blocks<T, SlabStream<T, true>>(pool, aux, perm, stride, m, count, rhs, z);
 }
 
 // The diagonal squares of the slabs of `count` FP64 blocks, in place: the unit lower triangle's inverse below the
 // diagonal, the upper triangle's on and above it.  One warp per square; lane j computes column j of both
 // by substitution in FP64 registers, the triangles read from shared memory as broadcasts.  Bound by those
 // reads and the FMAs: 141 us for 2,250 blocks of 324, whose factorisation takes 8.9 ms.
+//
+// A triangle T stays as it is (kept) where max|T| max|T^-1| is above INVERT_BOUND or not finite, or where either lies
+// so far from 1 that products with the inverse could leave the normal range.  The residual of y = X b for a
+// computed inverse X is of the order eps |T| |X| |b|, against eps |T| |y| by substitution: with triangles below 128
+// the normwise backward error of random, graded and near-singular blocks of 32 to 100 rows stayed below 8 % of
+// 8 m eps, at 256 to 1,024 it came to 46 %, above to any multiple of it.  The triangles of the solver's own cells
+// and faces (degrees 0 to 8, CFL 1 to 50) lie at 2 to 12 in the median and at 70 (cells) and 153 (a face) at most.
 constexpr int SQUARE_WARPS = 4, SQUARE_PITCH = 33;
-__global__ void __launch_bounds__(32 * SQUARE_WARPS)
-k_slab_invert(double *__restrict__ pool, size_t stride, int m, int count) {
+constexpr double INVERT_BOUND = 128, INVERT_RANGE = 0x1p900;
+// Largest entries by their high words, which order |v| and put infinities and NaN last.
+__device__ __forceinline__ void most(unsigned &mx, double v) { mx = max(mx, (unsigned)__double2hiint(v) & 0x7fffffffu); }
+__device__ __forceinline__ bool invertible(unsigned t_hi, unsigned x_hi) {  // the lanes' largest |T| and |T^-1|
+    const double t = __hiloint2double((int)__reduce_max_sync(0xffffffffu, t_hi), -1);
+    const double x = __hiloint2double((int)__reduce_max_sync(0xffffffffu, x_hi), -1);
+    return t <= INVERT_RANGE && x <= INVERT_RANGE && t * x <= INVERT_BOUND;
+}
+__global__ void __launch_bounds__(32 * SQUARE_WARPS, 4)
+k_slab_invert(double *__restrict__ pool, size_t stride, int m, int count, unsigned char *__restrict__ kept) {
     constexpr int W = 2;
     __shared__ double tile[SQUARE_WARPS][32 * SQUARE_PITCH + 32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, slabs = (m + 31) / 32;
@@ -585,11 +664,15 @@ k_slab_invert(double *__restrict__ pool, size_t stride, int m, int count) {
     const int s = (int)(job % slabs), r0 = 32 * s, nt = min(32, m - r0);
     double *a = tile[wib], *rd = a + 32 * SQUARE_PITCH;
     double *S = pool + (size_t)(job / slabs) * stride + (size_t)r0 * m + (size_t)r0 * nt;  // group r0 / W, row 0
+    // the largest entries of the lane's row (T) and column (T^-1) of L and U
+    unsigned tl = 0x3ff00000u, tu = 0, xl = 0x3ff00000u, xu = 0;  // (L: its unit diagonal)
     for (int g = 0; g < 32 / W; ++g)
 #pragma unroll
         for (int w = 0; w < W; ++w) {
             const int c = g * W + w;
-            a[lane * SQUARE_PITCH + c] = lane < nt && c < nt ? S[((size_t)g * nt + lane) * W + w] : lane == c ? 1. : 0.;
+            const double v = lane < nt && c < nt ? S[((size_t)g * nt + lane) * W + w] : lane == c ? 1. : 0.;
+            a[lane * SQUARE_PITCH + c] = v;
+            if (lane < nt && c < nt) most(c < lane ? tl : tu, v);
         }
     rd[lane] = 1. / a[lane * SQUARE_PITCH + lane];
     __syncwarp();
@@ -600,10 +683,13 @@ k_slab_invert(double *__restrict__ pool, size_t stride, int m, int count) {
     for (int k = 0; k < 31; ++k)
 #pragma unroll
         for (int i = k + 1; i < 32; ++i) x[i] = fma(-a[i * SQUARE_PITCH + k], x[k], x[i]);
+#pragma unroll
+    for (int i = 1; i < 32; ++i) most(xl, x[i]);
+    const bool inv_l = invertible(tl, xl);
     __syncwarp();
 #pragma unroll
     for (int i = 1; i < 32; ++i)
-        if (i > lane) a[i * SQUARE_PITCH + lane] = x[i];
+        if (i > lane && inv_l) a[i * SQUARE_PITCH + lane] = x[i];
 #pragma unroll
     for (int i = 0; i < 32; ++i) x[i] = i == lane ? 1. : 0.;
 #pragma unroll
@@ -612,15 +698,20 @@ k_slab_invert(double *__restrict__ pool, size_t stride, int m, int count) {
 #pragma unroll
         for (int i = 0; i < k; ++i) x[i] = fma(-a[i * SQUARE_PITCH + k], x[k], x[i]);
     }
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+        if (lane < nt) most(xu, x[i]);
+    const bool inv_u = invertible(tu, xu);
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-        if (i <= lane) a[i * SQUARE_PITCH + lane] = x[i];
+        if (i <= lane && inv_u) a[i * SQUARE_PITCH + lane] = x[i];
     __syncwarp();
-    if (lane < nt)
+    if (lane < nt && (inv_l || inv_u))
         for (int g = 0; g < nt / W; ++g)
 #pragma unroll
             for (int w = 0; w < W; ++w) S[((size_t)g * nt + lane) * W + w] = a[lane * SQUARE_PITCH + g * W + w];
+    if (lane == 0) kept[job] = (inv_l ? 0 : KEPT_L) | (inv_u ? 0 : KEPT_U);
 }
 
 }  // namespace dgh

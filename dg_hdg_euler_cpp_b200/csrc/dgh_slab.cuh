@@ -11,6 +11,9 @@ namespace dgh {
 // 32 s m + (j / W) nt W + i W + j % W.  Lane i of a warp then loads its row's next W columns as
 // one 16-byte vector, and the warp's load of a column group is nt*16 contiguous bytes.
 // m = 4n^2 (cells) and 4n (faces) are multiples of W, so every group is complete.
+// The 32 x 32 diagonal squares of FP64 slabs hold L^{-1} and U^{-1} in place of the triangles, but for
+// those that are marked as kept (k_slab_invert); FP32 and FP16 slabs hold the triangles themselves.
+__host__ __device__ constexpr int slab_count(int m) { return (m + 31) / 32; }
 template <typename T> struct SlabVec;
 template <> struct SlabVec<double> {
     using V = double2;
