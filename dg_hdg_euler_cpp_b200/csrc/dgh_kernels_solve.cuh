@@ -122,6 +122,12 @@ __device__ __forceinline__ void slab_fma(const uint4 &v, const float *y, unsigne
     acc = add2(acc, d);
 }
 
+// FP32 blocks at least this wide fetch of a diagonal square only the triangle of the sweep, L going forward and
+// U going back: fetched whole in both sweeps, the squares add a tenth to the bytes of 324-wide blocks.  65,536
+// blocks of 324 (256, 144): 4.77 (2.71, 0.91) ms, with whole squares 5.06 (2.88, 0.98); 4,096 of 100: 55 against
+// 53 us, where the bytes do not bound it.  (FP16, bound by instructions: 3 to 6 % slower at 100 to 196.)
+constexpr int HALF_SQUARES = 128;
+
 __device__ __forceinline__ void ring_copy(unsigned dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -130,7 +136,8 @@ __device__ __forceinline__ void ring_copy(unsigned dst, const void *src) {
 // a slab's chunks ascending (sweep 0) or descending, so that the diagonal's come last in a slab, or,
 // transposed, first.  Chunk j of slab s lies at its offset in memory and in its ring slot alike (group by
 // group, row by row), and unit i of its 16-byte units is copied by lane i % 32.
-template <typename T, bool TRANS> struct SlabStream {
+// HALF (D = 1): of a diagonal square only the triangle of the sweep.
+template <typename T, bool TRANS, bool HALF = false> struct SlabStream {
     using S = SolveType<T>;
     static constexpr int D = 32 / S::CW, UNITS = S::CW / S::W;  // chunks in a diagonal square, groups in a chunk
     static constexpr int STAGES = S::STAGES + TRANS;
@@ -157,7 +164,12 @@ template <typename T, bool TRANS> struct SlabStream {
         if (blk < count) {
             const unsigned dst = base + fill_at + (threadIdx.x & 31) * 16;
             const bool rows = s < slabs - 1 || m % 32 == 0;
-            if (rows && j != ragged) {
+            if (HALF && rows && j == s) {  // the triangle that the sweep reads
+                const int r = threadIdx.x & 31;
+#pragma unroll
+                for (int u = 0; u < UNITS; ++u)
+                    if (dir == 0 ? r >= u * S::W : r < (u + 1) * S::W) ring_copy(dst + u * 512, src + u * 32);
+            } else if (rows && j != ragged) {
 #pragma unroll
                 for (int u = 0; u < UNITS; ++u) ring_copy(dst + u * 512, src + u * 32);
             } else {
@@ -503,6 +515,8 @@ __device__ __forceinline__ void lu_solve_body(int bx, int G, const T *__restrict
                                               const int *__restrict__ perm, size_t stride, int m, int count,
                                               const double *__restrict__ rhs, double *__restrict__ z) {
     if (solve_whole<T>(m)) lu_solve_blocks<T, SlabWhole<T, false>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
+    else if (sizeof(T) == 4 && m >= HALF_SQUARES)
+        lu_solve_blocks<T, SlabStream<T, false, sizeof(T) == 4>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
     else lu_solve_blocks<T, SlabStream<T, false>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
 }
 template <typename T>
