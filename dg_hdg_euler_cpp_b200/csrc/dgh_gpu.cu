@@ -2071,6 +2071,7 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
         k_fill_trace_mass<<<(unsigned)((c->NT + tb - 1) / tb), tb, 0, c->stream>>>(c->inv_trace_mass, c->basis, c->g, n, c->NT);
         c->launched(2);
         const size_t tsz = c->mixed() ? sizeof(float) : sizeof(double);
+        if (c->has_dg() || c->has_hdg()) c->lu_grid = c->sms * lu_resident(c->m, c->has_hdg());
         if (c->has_dg() && c->ilu2d()) {  // block ILU(0) factors instead of the block-Jacobi pool
             c->dg_perm = c->alloc<int>((size_t)c->cells * c->m);
         } else if (c->has_dg()) {
@@ -2096,11 +2097,17 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
             c->Y = c->alloc<double>((size_t)c->cells * c->m);
             c->cy = c->alloc<double>((size_t)c->cells * c->t);
             c->hrhs = c->alloc<double>(c->NT);
-            // [A | B | r | pad] and, where X is not kept, the solved columns
-            const size_t per_cell = (size_t)c->m * (lu_aug_ld(c->m, c->t) + (c->c32() ? c->t : 0)) * sizeof(double);
-            const size_t budget = (size_t)8 << 30;  // condensation workspace: at most 8 GiB
+            // condensation workspace, at most 8 GiB: [A | B | r | pad], of the FP32 condensation in FP32.  Its
+            // FP64 form, whose matrices and solved columns take 2.6 times that at k = 8, takes the cells in as
+            // many chunks as that needs (aug_chunk), but has room for a cell per resident LU CTA: a mesh
+            // of fewer cells is one chunk, since each would take as long as all of them
+            const size_t row = lu_aug_ld(c->m, c->t);
+            const size_t per_cell = (size_t)c->m * row * (c->c32() ? sizeof(float) : sizeof(double));
+            const size_t budget = (size_t)8 << 30;
             c->aug_cells = (int)std::max<size_t>(1, std::min<size_t>(c->cells, budget / per_cell));
             c->aug_bytes = (size_t)c->aug_cells * per_cell;
+            if (c->c32())
+                c->aug_bytes = std::max(c->aug_bytes, std::min(c->cells, c->lu_grid) * c->m * (row + c->t) * sizeof(double));
             c->aug = reinterpret_cast<double *>(c->alloc<char>(c->aug_bytes));
             if (c->c32()) c->aug32 = reinterpret_cast<float *>(c->aug);
             c->aug_perm = c->alloc<int>((size_t)c->aug_cells * c->m);
@@ -2134,9 +2141,6 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
                 c->dg_slot_count = std::min(c->cells, c->sms * lu_fused_resident(c->n));
                 c->dg_slots = c->alloc<double>((size_t)c->dg_slot_count * c->m * c->m);
             }
-        }
-        if (c->has_dg() || c->has_hdg()) {
-            c->lu_grid = c->sms * lu_resident(c->m, c->has_hdg());
         }
         if (c->has_dg() && c->ilu2d()) ilu2_build(c);
         if (c->slabbed()) c->slab.buf = c->alloc<double>(16);
@@ -2739,10 +2743,11 @@ void hdg_condense_chunk(dgh_ctx *c, int variant, const double *r, int first, int
     c->launched();
 }
 // Cells per chunk of the FP32-storage condensation's workspace: augmented matrices of element type T
-// and, in the FP64 form, their solved columns X.
+// and, in the FP64 form, their solved columns X; of several chunks, whole rounds of the LU's resident CTAs.
 template <typename T> int aug_chunk(const dgh_ctx *c) {
     const size_t row = lu_aug_ld(c->m, c->t) + (sizeof(T) == 8 ? c->t : 0);
-    return (int)std::max<size_t>(1, std::min<size_t>(c->cells, c->aug_bytes / ((size_t)c->m * row * sizeof(T))));
+    const int n = (int)std::max<size_t>(1, std::min<size_t>(c->cells, c->aug_bytes / ((size_t)c->m * row * sizeof(T))));
+    return sizeof(T) == 8 && n < c->cells && n > c->lu_grid ? n - n % c->lu_grid : n;
 }
 // FP32-storage condensation of cells [first, first + count), variant 0: [A | B | r] assembled in
 // FP64, the LU on the FP64 tensor pipe with the fused right-hand-side solve (X behind the matrices
