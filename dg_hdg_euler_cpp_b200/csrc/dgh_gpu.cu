@@ -2836,12 +2836,14 @@ template <class F> int tune_pick(dgh_ctx *c, F &&f, double *ms_out) {
     ms_out[1] = best[1];
     return best[1] < best[0] ? 1 : 0;
 }
-// The cached or newly tuned variant of one kind (0 DG blocks, 1 FP64 condensation, 2 FP32-storage
-// condensation, 3 the DG block solve's grid shape, which also depends on the block count, 4 the
-// fused DG factorisation's CTAs per SM, variant v = v + 1 CTAs).
+// The cached or newly tuned variant of one kind (0 DG blocks, whose variant 0 is another path under the
+// over-integrated rule, 1 FP64 condensation, 2 FP32-storage condensation, 3 the DG block solve's grid shape
+// and 4 the fused DG factorisation's CTAs per SM, variant v = v + 1 CTAs, which also depend on the block count).
 template <class F> int tuned_variant(dgh_ctx *c, int kind, F &&time_both, double *ms_out) {
     if (!c->cfg.autotune) return 0;
-    const auto key = std::make_tuple(kind, c->n, c->cfg.precision, kind == 3 ? c->cells : 0);
+    if (kind == 4 && c->dg_slot_count <= c->sms) return 1;  // the same grid either way: nothing to time
+    const int mesh = kind == 3 || kind == 4 ? c->cells : kind == 0 && c->overint() ? 1 : 0;
+    const auto key = std::make_tuple(kind, c->n, c->cfg.precision, mesh);
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
@@ -2945,7 +2947,7 @@ int dgh_block_jacobi_refresh(dgh_ctx *c, int op) {
                 c->dg_variant = tuned_variant_all(c, 0, [&](int v) { dg_factor(c, v, 0, sample); }, c->tune_ms);
                 c->check_status();
             }
-            if (c->fused_ctas < 0) {  // the fused path's residency (kind 4): 1 or 2 CTAs per SM
+            if (c->fused_ctas < 0) {  // the fused path's residency (kind 4): one CTA per SM or all
                 const bool fused = (c->half16() || c->dg_variant == 0) && !c->overint();
                 if (fused) {
                     const int sample = std::min(c->cells, std::max(c->lu_grid, 1) * 4);

@@ -203,7 +203,8 @@ int dgh_gmres(dgh_ctx *ctx, int op, const double *rhs, double *x, int limit, dou
 /* Per-degree autotuner (no counterpart in the reference).  With dgh_config.autotune set, the
  * first DG block-Jacobi refresh and the first HDG condensation of a context time their
  * factorisation variants on a sample of the context's own cells and keep the faster one; the
- * choice is cached per (degree, precision) for the process.  Variants: DG blocks 0 = FP64
+ * choice is cached per (degree, precision) for the process, of the DG blocks apart for the
+ * over-integrated rule.  Variants: DG blocks 0 = FP64
  * LU on the tensor pipe (FP32 slabs in the mixed form), 1 = right-looking LU (FP32 in the
  * mixed form); condensation 0 = tensor-pipe LU with the fused right-hand-side solve,
  * 1 = right-looking LU then the tensor-pipe back substitution.  All variants compute the same
@@ -217,7 +218,8 @@ int dgh_autotune_report(const dgh_ctx *ctx, double out[6]);
  * shares); timed at the first DG refresh on the context's own factors, cached per (degree,
  * precision, cell count); default 0.  DGH_SHAPE_FUSED_CTAS: CTAs per SM of the fused
  * DG factorisation, 1 (each CTA's FP64 slot fits L2) or 2 (every CTA that is resident); timed at
- * the first DG refresh on a sample of the cells, cached per (degree, precision); default 2.
+ * the first DG refresh on a sample of the cells, cached per (degree, precision, cell count), and not
+ * timed where a mesh has no cell for a second CTA; default 2.
  * dgh_shape_set fixes a shape instead; every shape computes the same bits.
  * dgh_autotune_shapes: out[0] = the solve grid shape in use (-1 before the first DG refresh),
  * out[1..2] its tuning times (ms) for shapes 0 and 1; out[3] = the fused CTAs per SM in use
