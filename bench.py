@@ -14,8 +14,9 @@ warm-up update), updates 2-4 timed.  Per configuration (method x precision):
 value = (K_dg + K_hdg) / (t_dg + t_hdg) over the fastest reduced-precision DG form and the
 fastest reduced-precision HDG form that keep the reference's linear tolerance (FORMS below,
 forcing 0); the same over the forms that may also stop at the acceptance round-off floor is
-"with_forcing_floor".  The FP64 forms and the per-form numbers are in "breakdown", and each
-reduced form's speed-up, state error and Krylov change against FP64 at the top level.  e2e
+"with_forcing_floor".  The FP64 forms and the per-form numbers are in "breakdown", which is part of the
+whole record on stderr only; each reduced form's speed-up, state error and Krylov change against
+FP64 are at the top level, in the one line on stdout.  e2e
 repeats the headline forms' timed updates through the C ABI with host buffers
 (dgh_newton_update_host: state H2D, update, state D2H every step).
 
@@ -752,6 +753,26 @@ def cpu_baseline(args) -> dict:
             "all_core": allc}
 
 
+def result_line(record: dict) -> str:
+    """The one line on stdout: the record without its breakdown and without the CPU baseline's
+    per-process samples, floats to nine digits, some 5,000 characters (a caller that keeps the end of
+    the output lost the start of a whole record).  The whole record goes to stderr."""
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.9g}")
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items()}
+        return [short(x) for x in v] if isinstance(v, (list, tuple)) else v
+
+    out = short({k: v for k, v in record.items() if k != "breakdown"})
+    cpu = out.get("cpu_baseline")
+    if cpu:
+        out["cpu_baseline"] = {k: v for k, v in cpu.items() if k != "all_core"} | {
+            "single_thread": {k: cpu["single_thread"][k] for k in ("value", "unit", "cores")},
+            "host": cpu["all_core"]["host"], "wall_s": cpu["all_core"]["wall_s"]}
+    return json.dumps(out)
+
+
 def main():
     args = parse()
     if args.impl == "reference":
@@ -882,7 +903,8 @@ def main():
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(args)
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(result_line(line), flush=True)
     if comm is not None:
         comm.close()
     if pg is not None:
