@@ -348,8 +348,7 @@ struct dgh_lockstep {
         size_t smem = 0;
     };
     std::vector<Range> degrees;  // operator launches (J·v or Schur apply): key = n (nodes per direction)
-    // block-Jacobi launches: key 0 FP64 LU, 1 FP32 LU, 2 FP32 LU narrow (m < 64), 3 FP16 LU,
-    // 4 FP32 inverses (HDG face blocks); for HDG groups re-planned every session
+    // block-Jacobi launches: key LsLayout; for HDG groups re-planned every session
     std::vector<Range> layouts;
     std::vector<int> layout_keys;  // the keys the captured cycle graph was built with
     int red_total = 0;
@@ -1267,14 +1266,20 @@ void gmres(dgh_ctx *c, int op, const double *rhs, double *x, int limit, double t
 }
 
 // ---- lockstep batch of DG GMRES solves ----------------------------------------------------------
+// Factor layouts of a batched solve, a launch each.  FP32 blocks that are held whole (up to 64 wide, 66 KB of shared
+// memory a CTA) and streamed ones (up to 43 KB) do not share one: the streamed ones would lose residency by it.
+enum LsLayout { LS_FP64, LS_FP32_WHOLE, LS_FP32, LS_FP16, LS_INVERSE };
+int ls_layout(bool half16, bool mixed, int m) {
+    return half16 ? LS_FP16 : !mixed ? LS_FP64 : solve_whole<float>(m) ? LS_FP32_WHOLE : LS_FP32;
+}
 // The block solves z = M^{-1} src of every gated member, one launch per factor layout.
 void ls_solve_all(dgh_lockstep *L, int src, int dst, int j, int gate) {
     for (const auto &r : L->layouts) {
-        if (r.key == 0)
+        if (r.key == LS_FP64)
             k_ls_solve<double><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
-        else if (r.key == 1 || r.key == 2)
+        else if (r.key == LS_FP32_WHOLE || r.key == LS_FP32)
             k_ls_solve<float><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
-        else if (r.key == 3)
+        else if (r.key == LS_FP16)
             k_ls_solve<__half><<<r.blocks, SOLVE_THREADS, r.smem, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
         else
             k_ls_inv_apply<<<r.blocks, INV_APPLY_THREADS, 0, L->stream>>>(L->table, r.first, r.count, src, dst, j, gate);
@@ -1300,17 +1305,32 @@ void ls_jv_all(dgh_lockstep *L, int src, int dst, int gate) {
         L->launched(2);
     }
 }
-// A member's CTAs in a batched solve: no more than are resident, so that a warp's ring runs on from block
-// to block.
-int ls_solve_blocks(const dgh_ctx *c, int count) { return solve_grid(c, count, SOLVE_WARPS, 5, 0); }
-// Dynamic shared memory of the block solve of factor layout `key` (0 FP64, 1 and 2 FP32, 3 FP16).
-size_t ls_solve_smem(int key, int m) {
-    const size_t warp = key == 0 ? solve_warp_bytes<double>(m) : key == 3 ? solve_warp_bytes<__half>(m) : solve_warp_bytes<float>(m);
-    const void *fn = key == 0 ? (const void *)k_ls_solve<double>
-                     : key == 3 ? (const void *)k_ls_solve<__half>
-                                : (const void *)k_ls_solve<float>;
-    allow_dynamic_smem(fn, SOLVE_WARPS * warp);
-    return SOLVE_WARPS * warp;
+// The grid and shared memory of a batched solve, from its members' widths and block counts (L->host).  The
+// launch's shared memory is its widest member's.  A member takes no more CTAs than are resident with that, so that a
+// warp's ring runs on from block to block, and no more than 5 an SM (FP16, of which 6 fit, takes about
+// 1 % longer for a batch of k = 2, 4, 8 with 6).  The members' CTAs together are left to the scheduler: shares set beforehand
+// would have to foresee the members' times.
+void ls_plan_solve(dgh_lockstep *L, dgh_lockstep::Range &r) {
+    const dgh_ctx *c = L->members[r.first];
+    r.blocks = 0;
+    r.smem = 0;
+    int resident = 1;
+    auto fit = [&](auto tag) {
+        using T = decltype(tag);
+        for (int i = r.first; i < r.first + r.count; ++i)
+            r.smem = std::max(r.smem, SOLVE_WARPS * solve_warp_bytes<T>(L->host[i].m));
+        allow_dynamic_smem((const void *)k_ls_solve<T>, r.smem);
+        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_ls_solve<T>, SOLVE_THREADS, r.smem), "occupancy");
+    };
+    if (r.key == LS_FP64) fit(double());
+    else if (r.key == LS_FP16) fit(__half());
+    else if (r.key != LS_INVERSE) fit(float());
+    constexpr int inv_wpc = INV_APPLY_THREADS / 32;
+    for (int i = r.first; i < r.first + r.count; ++i) {
+        L->host[i].solve0 = r.blocks;
+        r.blocks += r.key == LS_INVERSE ? (L->host[i].cells + inv_wpc - 1) / inv_wpc
+                                        : solve_grid(c, L->host[i].cells, SOLVE_WARPS, std::min(resident, 5), 0);
+    }
 }
 // The HDG members' face-block Jacobi launches from their current state (FP32 inverses or LU
 // factors, chosen at each refresh): consecutive members with the same form share a launch.
@@ -1319,7 +1339,7 @@ void ls_plan_face_precond(dgh_lockstep *L) {
     std::vector<int> keys;
     for (int i = 0; i < (int)L->members.size(); ++i) {
         const dgh_ctx *c = L->members[i];
-        const int key = c->face_inverse ? 4 : c->mixed() ? 2 : 0;
+        const int key = c->face_inverse ? LS_INVERSE : ls_layout(false, c->mixed(), c->fw);
         keys.push_back(key);
         if (L->layouts.empty() || L->layouts.back().key != key) {
             dgh_lockstep::Range r;
@@ -1327,16 +1347,12 @@ void ls_plan_face_precond(dgh_lockstep *L) {
             r.key = key;
             L->layouts.push_back(r);
         }
-        auto &lr = L->layouts.back();
-        L->host[i].solve0 = lr.blocks;
+        ++L->layouts.back().count;
         L->host[i].pool = c->face_pool;
         L->host[i].perm = c->face_perm;
         L->host[i].kept = c->face_kept;
-        constexpr int inv_wpc = INV_APPLY_THREADS / 32;
-        lr.blocks += key == 4 ? (c->faces + inv_wpc - 1) / inv_wpc : ls_solve_blocks(c, c->faces);
-        ++lr.count;
-        if (key != 4) lr.smem = std::max(lr.smem, ls_solve_smem(key, c->fw));
     }
+    for (auto &r : L->layouts) ls_plan_solve(L, r);
     if (keys != L->layout_keys && L->cycle) {  // a different launch plan: capture the cycle again
         ck(cudaGraphExecDestroy(L->cycle), "cudaGraphExecDestroy");
         L->cycle = nullptr;
@@ -3446,7 +3462,6 @@ int dgh_lockstep_create_op(dgh_ctx *const *members, int count, int op, dgh_locks
             ck(cudaMallocHost(&L->host, sizeof(LsMember) * count), "cudaMallocHost");
             ck(cudaMallocHost(&L->flags_host, sizeof(int) * count), "cudaMallocHost");
             ck(cudaMallocHost(&L->tails_host, sizeof(LsTail) * count), "cudaMallocHost");
-            auto layout_of = [&](const dgh_ctx *c) { return c->half16() ? 3 : !c->mixed() ? 0 : c->m < 64 ? 2 : 1; };
             for (int i = 0; i < count; ++i) {
                 dgh_ctx *c = L->members[i];
                 LsMember &t = L->host[i];
@@ -3503,19 +3518,16 @@ int dgh_lockstep_create_op(dgh_ctx *const *members, int count, int op, dgh_locks
                 int cpb = 1;
                 DGH_DISPATCH_N(c->n, { cpb = Team<N>::CPB; });
                 dr.blocks += c->team_blocks(cpb);
-                const int key = layout_of(c);
+                const int key = ls_layout(c->half16(), c->mixed(), c->m);
                 if (L->layouts.empty() || L->layouts.back().key != key) {
                     dgh_lockstep::Range r;
                     r.first = i;
                     r.key = key;
                     L->layouts.push_back(r);
                 }
-                auto &lr = L->layouts.back();
-                t.solve0 = lr.blocks;
-                lr.blocks += ls_solve_blocks(c, c->cells);
-                ++lr.count;
-                lr.smem = std::max(lr.smem, ls_solve_smem(key, c->m));
+                ++L->layouts.back().count;
             }
+            for (auto &r : L->layouts) ls_plan_solve(L, r);
             for (const auto &r : L->layouts)
                 for (const auto &q : L->layouts)
                     if (&r != &q && r.key == q.key) fail(DGH_ERR_INVALID, "lockstep factor layouts are not contiguous");
