@@ -344,6 +344,20 @@ __device__ __forceinline__ float4 square_four(const uint4 *base, int nt, int r, 
 __device__ __forceinline__ float4 square_four(const uint4 *base, int nt, int r, int c, const float *) {
     return *reinterpret_cast<const float4 *>(base + (c >> 2) * nt + r);
 }
+// A triangle with a subnormal diagonal entry, whose reciprocal may be out of range: true quotients, a column at a
+// time, ascending or descending.  at(r, c): the triangle's entries.
+template <bool ASC, class At> __device__ __forceinline__ float triangle_divided(float t, int lane, int nt, const At &at) {
+#pragma unroll 1
+    for (int k = 0; k < nt; ++k) {
+        const int c = ASC ? k : nt - 1 - k;
+        const float e = lane < nt && (ASC ? lane >= c : lane <= c) ? at(lane, c) : 1.f;
+        if (lane == c) t = t / e;
+        const float y = __shfl_sync(0xffffffffu, t, c);
+        if (lane < nt && (ASC ? lane > c : lane < c)) t = fmaf(-e, y, t);
+    }
+    return t;
+}
+__device__ __forceinline__ bool any_subnormal(float d) { return __any_sync(0xffffffffu, fabsf(d) < 0x1p-126f); }
 // The slab's triangle: L (dir 0) or U (dir 1), lane i holding row i's right-hand side.
 template <typename T> __device__ __forceinline__ float slab_triangle(const uint4 *base, int lane, int nt, int dir, float t) {
     constexpr int W = SolveType<T>::W;
@@ -361,7 +375,10 @@ template <typename T> __device__ __forceinline__ float slab_triangle(const uint4
     };
     auto four = [&](int r, int c) { return square_four(base, nt, r, c, tag); };
     if (dir == 0) return triangle<true, true, false>(t, lane, nt, 1.f, own, four);
-    return triangle<false, false, sizeof(T) == 4>(t, lane, nt, lane < nt ? square_at(base, nt, lane, lane, tag) : 1.f, own, four);
+    const float d = lane < nt ? square_at(base, nt, lane, lane, tag) : 1.f;
+    if (sizeof(T) == 4 && any_subnormal(d))
+        return triangle_divided<false>(t, lane, nt, [&](int r, int c) { return square_at(base, nt, r, c, tag); });
+    return triangle<false, false, sizeof(T) == 4>(t, lane, nt, d, own, four);
 }
 // The same transposed: U^T (dir 0, lower) or L^T (dir 1, unit upper).
 __device__ __forceinline__ float slab_triangle_t(const uint4 *base, int lane, int nt, int dir, float t) {
@@ -373,7 +390,9 @@ __device__ __forceinline__ float slab_triangle_t(const uint4 *base, int lane, in
                            square_at(base, nt, c + 3, r, tag));
     };
     if (dir == 1) return triangle<false, true, false>(t, lane, nt, 1.f, own, four);
-    return triangle<true, false, true>(t, lane, nt, square_at(base, nt, col, col, tag), own, four);
+    const float d = square_at(base, nt, col, col, tag);
+    if (any_subnormal(d)) return triangle_divided<true>(t, lane, nt, [&](int r, int c) { return square_at(base, nt, c, r, tag); });
+    return triangle<true, false, true>(t, lane, nt, d, own, four);
 }
 
 // Squares of FP64 factors whose triangle is kept (k_slab_invert): a byte per square, slab by slab.

@@ -97,3 +97,22 @@ def test_cell_blocks_of_a_rough_linearisation(k):
             sl = slice(cell * m, (cell + 1) * m)
             assert backward_error(a.T if op == "dg_t" else a, x[sl], b[sl]) <= 8 * m * EPS, (op, cell)
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [4, 12, 28, 32])
+def test_fp32_factors_in_the_subnormal_range(width):
+    """FP32 factors of blocks around 1e-40, in steps of 2^-149: 2^-16 of the largest entry, so that a solve by
+    quotients keeps a backward error of 8 m 2^-16; a reciprocal of such a pivot is out of range."""
+    from dg_hdg_euler_cpp_b200.solver import BlockJacobi
+
+    count = 6
+    rng = np.random.default_rng(width)
+    a = 1e-40 * rng.uniform(-1, 1, size=(count, width, width))
+    b = 1e-40 * rng.uniform(-1, 1, size=(count, width))
+    bj = BlockJacobi(width, count, "mixed", 0)
+    bj.factor(a)
+    x = bj.apply(b.reshape(-1)).reshape(count, width)
+    bj.close()
+    for i in range(count):
+        assert backward_error(a[i], x[i], b[i]) <= 8 * width * 2.0**-16, i
