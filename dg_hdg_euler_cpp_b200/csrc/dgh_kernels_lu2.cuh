@@ -60,8 +60,14 @@ __host__ __device__ constexpr int cr_warps(int m) {
     return m <= 32 ? 1 : m <= 64 ? 2 : m <= 128 ? 4 : m <= 160 ? 5 : m <= 224 ? 7 : m <= 384 ? 8 : 16;
 }
 __host__ __device__ constexpr int cr_rows(int warps) { return warps == 8 ? 2 : 1; }
+// CTAs per SM that the registers are cut for (128 to 170 a thread): the most that leave the tiles without spills
+// of any size and their loads in flight.  One step more (16, 8, 4, 3 CTAs of 1, 2, 5, 7 warps) spills up to 336 bytes a
+// thread or cuts the loads: LU of 12,800 blocks of 64 1.38 against 1.22 ms, augmented 2.88 against 2.26; 5,913 of 144
+// 3.14, 3.09 and 5.76, 5.53; 4,087 of 196 5.05, 4.53 and 8.66, 7.90.  One step less for 4 warps (3): 10,201 of 100
+// 2.87, 2.82, but 4,096, which are 10 rounds in place of 7, 1.15 and 1.21; two less (2, of 5 warps too) 3.45 and, 144
+// wide, 3.61.
 template <int NW> constexpr int cr_min_ctas() {
-    return NW == 1 ? 16 : NW == 2 ? 8 : NW <= 5 ? 4 : NW == 7 ? 3 : NW <= 11 ? 2 : 1;
+    return NW == 1 ? 12 : NW == 2 ? 6 : NW == 4 ? 4 : NW == 5 ? 3 : NW <= 8 ? 2 : 1;
 }
 __host__ __device__ constexpr int cr_stage_pitch(int m) { return m + (18 - m % 16) % 16; }
 __host__ __device__ constexpr int cr_area(int m) {  // doubles of the panel / staging area
