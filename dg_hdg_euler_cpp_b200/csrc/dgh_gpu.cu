@@ -2038,7 +2038,7 @@ int create_ctx(const dgh_config *cfg, const SlabInit *slab, dgh_ctx **out) {
         c->traces = c->alloc<double>((size_t)c->cells * NFACES * n * NVAR);
         c->traces2 = c->alloc<double>((size_t)c->cells * NFACES * n * NVAR);
         c->size_sweeps();
-    c->partial = c->alloc<double>((size_t)std::max<long long>(KR_MAXK * c->red_grid, 4LL * c->cells + 64));
+        c->partial = c->alloc<double>((size_t)std::max<long long>(KR_MAXK * c->red_grid, 4LL * c->cells + 64));
         c->red = c->alloc<double>(4 * KR_MAXK);
         c->vol = c->alloc<double>((size_t)c->cells * c->P * 3);
         c->fcache = c->alloc<double>((size_t)c->faces * n * 8);
@@ -3230,7 +3230,7 @@ const double *dgh_gmres_residual(dgh_ctx *c, int op) {
 // ---- Standalone block Jacobi (BlockJacobi, block_jacobi.hpp:7-47) -----------------------------------
 // A pool of `count` dense m x m blocks, factored by one of the device LU kernels and applied as
 // z = A^{-1} x per block.  It runs on a bare context that carries only what the launch helpers
-// read: the stream, the status word, the SM count and the tensor-pipe kernel's scratch.
+// read: the stream, the status word and the SM count.
 struct dgh_block_jacobi {
     dgh_ctx *c = nullptr;
     int m = 0, count = 0, precision = 0, variant = 0;
@@ -3253,7 +3253,7 @@ int dgh_block_jacobi_create(int m, int count, int precision, int variant, int de
         need(m >= 1 && count >= 1 && m <= LU_MAX_WIDTH, "Invalid block size or count");
         need(precision == DGH_PRECISION_FP64 || precision == DGH_PRECISION_MIXED, "Invalid precision");
         need(variant >= 0 && variant <= 3, "Invalid factorisation variant");
-        need(variant != 0 || m % 4 == 0, "LU block width unsupported by the left-looking kernel");
+        need(variant != 0 || m % 4 == 0, "LU block width unsupported by the tensor-pipe kernel");
         need(variant < 2 || (m <= 64 && m % 4 == 0), "block width unsupported by the narrow LU");
         need(variant != 3 || precision == DGH_PRECISION_MIXED, "explicit inverses are the mixed form only");
         need(m % 4 == 0, "block width must be a multiple of 4 (slab layout)");

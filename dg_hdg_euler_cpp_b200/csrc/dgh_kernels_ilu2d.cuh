@@ -71,7 +71,7 @@ __global__ void k_copy_blocks(TF *const *__restrict__ dst, const TF *const *__re
     }
 }
 
-// [A_ii | I | 0] in FP64 (row length 2m + 1) from the stored diagonal blocks of the listed rows,
+// [A_ii | I | 0] in FP64 (row length lu_aug_ld(m, m)) from the stored diagonal blocks of the listed rows,
 // for the augmented LU's solve: X = A_ii^{-1}.
 template <typename TF>
 __global__ void k_ilu_stage_inverse(double *__restrict__ aug, const TF *__restrict__ diag, const int *__restrict__ rows,

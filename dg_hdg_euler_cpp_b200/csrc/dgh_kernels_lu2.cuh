@@ -12,9 +12,9 @@
 // come out as L^{-1} P [B | r] and only the back substitution (cr_back) remains.
 //
 // What bounds it: at m = 324 two matrices fit an SM (shared memory), and their chains of panel
-// latencies (about 1100 cycles a column with both running) leave the FP64 pipe 27 % busy; small
-// widths run many CTAs per SM.  Measured on one B200, LU of 2368 blocks of 324 (4096 of 100, 36):
-// 6.1 ms (0.73, 0.13) against 9.1 ms (2.41, 0.77) for the left-looking kernel; with 145 augmented
+// latencies (about 1100 cycles a column with both running) leave the FP64 tensor pipe 17 % busy (30 %
+// with augmented columns); small widths run many CTAs per SM.  Measured on one B200, LU of 2368 blocks
+// of 324 (4096 of 100, 36): 6.1 ms (0.73, 0.13) against 9.1 ms (2.41, 0.77) for the left-looking kernel; with 145 augmented
 // columns, 1776 of 324: 9.7 against 11.1 ms.
 //
 // Storage: every row of L and U stays in the ORIGINAL row of the matrix (row interchanges only
@@ -55,7 +55,7 @@ constexpr int CR_IP = 36;  // shared pitch of the 32 x 32 triangles (= 4 mod 16:
 constexpr int CR_PR = CR_H + 2;
 
 // Warps for width m, and panel rows a thread may hold: one thread per row where the registers of the
-// CTAs that fit an SM allow it (80 or more a thread), else two rows in the widest panels.
+// CTAs that fit an SM allow it, else two rows in the widest panels.
 __host__ __device__ constexpr int cr_warps(int m) {
     return m <= 32 ? 1 : m <= 64 ? 2 : m <= 128 ? 4 : m <= 160 ? 5 : m <= 224 ? 7 : m <= 384 ? 8 : 16;
 }

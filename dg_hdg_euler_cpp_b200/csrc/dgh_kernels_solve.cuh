@@ -20,8 +20,8 @@
 //  - a last slab of 4, 8 or 16 rows gives a row's column groups to 8, 4 or 2 lanes.
 // Measured inside solves, before (four 16-byte loads in flight, triangles solved from global memory) and now:
 // FP64, 4,096 blocks of 36: 36 and 16 us; 8,192 of 20: 40 and 15 us; 4,096 of 100, transposed: 126 and
-// 74 us; FP32, 5,917 blocks of 144: 131 and 97 us (5.1 TB/s); FP16, 65,536 blocks of 324: 2.68 and 2.54 ms
-// (5.7 TB/s).
+// 75 us; FP32, 5,917 blocks of 144: 131 and 92 us (5.3 TB/s), 65,536 of 324: 4.78 and 4.77 ms (5.8 TB/s); FP16,
+// 65,536 blocks of 324: 2.68 and 2.54 ms (5.7 TB/s), but 4,096, 1.15 rounds of warps, 200 and 207 us.
 #pragma once
 #include <type_traits>
 
@@ -673,7 +673,7 @@ k_lu_solve_t(const T *__restrict__ pool, const typename SolveType<T>::Aux *__res
 // The diagonal squares of the slabs of `count` FP64 blocks, in place: the unit lower triangle's inverse below the
 // diagonal, the upper triangle's on and above it.  One warp per square; lane j computes column j of both
 // by substitution in FP64 registers, the triangles read from shared memory as broadcasts.  Bound by those
-// reads and the FMAs: 141 us for 2,250 blocks of 324, whose factorisation takes 8.9 ms.
+// reads and the FMAs: 296 us for 4,096 blocks of 324, whose factorisation takes 15.6 ms.
 //
 // A triangle T stays as it is (kept) where max|T| max|T^-1| is above INVERT_BOUND or not finite, or where either lies
 // so far from 1 that products with the inverse could leave the normal range.  The residual of y = X b for a

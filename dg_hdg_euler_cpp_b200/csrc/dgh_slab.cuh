@@ -18,19 +18,11 @@ template <typename T> struct SlabVec;
 template <> struct SlabVec<double> {
     using V = double2;
     static constexpr int W = 2;
-    __device__ static double dot(const V &a, const double *y) { return a.x * y[0] + a.y * y[1]; }
-    __device__ static double dotv(const V &a, const V &y) { return a.x * y.x + a.y * y.y; }
 };
 template <> struct SlabVec<float> {
     using V = float4;
     static constexpr int W = 4;
-    __device__ static float dot(const V &a, const float *y) { return a.x * y[0] + a.y * y[1] + a.z * y[2] + a.w * y[3]; }
-    __device__ static float dotv(const V &a, const V &y) { return a.x * y.x + a.y * y.y + a.z * y.z + a.w * y.w; }
 };
-template <typename T> __device__ inline size_t slab_at(int nt, int i, int j) {
-    constexpr int W = SlabVec<T>::W;
-    return (size_t)(j / W) * nt * W + i * W + j % W;
-}
 
 // ---- 16-bit factor storage (the DG cell blocks, DGH_PRECISION_MIXED16) -------------------------
 // FP16 slabs with 8 columns per 16-byte group and rows padded to mp = m rounded up to 8 (zeros
