@@ -199,27 +199,29 @@ def algorithmic_bytes(kind: str, m: int, cells: int, fw: int, faces: int, t: int
     raise ValueError(kind)
 
 
-# DRAM bytes (read + write) of one k_lu_solve<float> launch per 324 x 324 block, from one ncu
-# capture at 64x64 k = 8 (4,096 blocks: 1.810513 GB read, 0.010409 GB written); the traffic of a
-# launch grows with the block count.
-SOLVE_FP32_TRAFFIC_PER_BLOCK_K8 = (1.810513e9 + 0.010409e9) / 4096
-# DRAM bytes of one k_lu_solve_half launch per block at k = 8: the DRAM throughput times the
-# duration of one launch at 64x64 k = 8 in one ncu capture (5.02 TB/s x 194.7 us over 4,096 blocks).
-SOLVE_HALF_TRAFFIC_PER_BLOCK_K8 = 5.02e12 * 194.7e-6 / 4096
+# DRAM bytes (read + written) of one k_lu_solve launch per 324 x 324 block, by the factors' storage, from one
+# ncu capture each at 64x64 k = 8 (4,096 blocks); the traffic of a launch grows with the block count.
+SOLVE_TRAFFIC_PER_BLOCK_K8 = {"float": (1.791855e9 + 0.011382e9) / 4096, "__half": (0.964909e9 + 0.012463e9) / 4096,
+                              "double": (3.782041e9 + 0.012984e9) / 4096}
+
+
+def solve_kernel(precision: str) -> str:
+    """The block solve of a DG form, as its record names it."""
+    storage = "__half" if precision.startswith("mixed16") else "double" if precision == "fp64" else "float"
+    return f"k_lu_solve<{storage}> (block-Jacobi solve, one launch per Krylov iteration)"
 
 
 def solve_traffic(args, kernel: str):
     """(DRAM bytes per launch of the dominant solve kernel at the bench's mesh, their source)."""
     if args.k != 8:
         return None, None
-    if kernel.startswith("k_lu_solve<float>"):
-        return (SOLVE_FP32_TRAFFIC_PER_BLOCK_K8 * args.nx * args.nx,
-                "ncu dram bytes of one launch at 64x64 k=8 (profiles/k_lu_solve_fp32_64x64_k8.md) times the "
-                "block-count ratio")
-    if kernel.startswith("k_lu_solve_half"):
-        return (SOLVE_HALF_TRAFFIC_PER_BLOCK_K8 * args.nx * args.nx,
-                "ncu DRAM throughput x duration of one launch at 64x64 k=8 "
-                "(profiles/k_lu_solve_half_and_hdg_apply32_64x64_k8.md) times the block-count ratio")
+    if kernel.startswith("k_lu_solve_half"):  # the FP16 solve's label in older records
+        kernel = solve_kernel("mixed16")
+    for storage, per_block in SOLVE_TRAFFIC_PER_BLOCK_K8.items():
+        if kernel.startswith(f"k_lu_solve<{storage}>"):
+            return (per_block * args.nx * args.nx,
+                    "ncu dram bytes of one launch at 64x64 k=8 (profiles/k_lu_solve_64x64_k8.md) times the block-count "
+                    "ratio")
     return None, None
 
 
@@ -322,9 +324,7 @@ def run_config(args, method: str, precision: str, torch, pg, peaks, sampler_on: 
     if method == "dg":
         kb = algorithmic_bytes("dg", s.block, s.cells, s.face_width, s.faces, s.local_trace, precision)
         tk = kernel_timers["precond"]
-        kernel = ("k_lu_solve_half (block-Jacobi solve from FP16 slabs" if precision.startswith("mixed16") else
-                  "k_lu_solve<%s> (block-Jacobi solve" % ("double" if precision == "fp64" else "float")) + \
-            ", one launch per Krylov iteration)"
+        kernel = solve_kernel(precision)
     else:
         kb = algorithmic_bytes("hdg_schur", s.block, s.cells, s.face_width, s.faces, s.local_trace,
                                "mixed" if FORMS[precision][1] else "fp64")

@@ -1,4 +1,5 @@
-"""bench.py's result line: complete, parseable and short, however long the breakdown is."""
+"""bench.py's result line: complete, parseable and short, however long the breakdown is; its kernels and their
+traffic are the present ones."""
 import json
 import sys
 
@@ -43,3 +44,22 @@ def test_result_line_is_short_and_complete():
         assert key in line, key
     assert abs(line["value"] - full["value"]) < 1e-9 and line["e2e"]["h2d_bytes_per_step"] == 169869312
     assert line["cpu_baseline"]["cores"] == 16 and line["cpu_baseline"]["single_thread"]["cores"] == 1
+
+
+def test_roofline_names_kernels_that_exist():
+    """Each DG form's solve is a kernel of the sources, with DRAM bytes from a committed capture: 1.0 to 1.1 times
+    the algorithmic bytes."""
+    import re
+    import types
+
+    sys.path.insert(0, str(ROOT))
+    import bench
+
+    sources = "".join(p.read_text() for p in (ROOT / "dg_hdg_euler_cpp_b200" / "csrc").glob("*.cu*"))
+    args = types.SimpleNamespace(k=8, nx=64)
+    for form in ("fp64", "mixed", "mixed16", "mixed-af", "mixed16-af"):
+        label = bench.solve_kernel(form)
+        assert re.search(r"^" + re.escape(label.split("<")[0]) + r"\(", sources, re.M), label
+        traffic, source = bench.solve_traffic(args, label)
+        assert 1.0 < traffic / bench.algorithmic_bytes("dg", 324, 4096, 36, 8192, 144, form) < 1.1, form
+        assert (ROOT / re.search(r"profiles/\S+\.md", source).group()).is_file(), source
