@@ -184,7 +184,7 @@ k_vol_apply_q_t(const double *__restrict__ w, const double *__restrict__ volq, d
     __shared__ BasisQ bq;
     for (int k = threadIdx.x; k < (int)(sizeof(BasisQ) / sizeof(double)); k += blockDim.x)
         reinterpret_cast<double *>(&bq)[k] = reinterpret_cast<const double *>(bqp)[k];
-    const int Q = bq.Q, QQ = Q * Q;
+    const int Q = bqp->Q, QQ = Q * Q;  // (bq is complete after the loop's first barrier only)
     const double sx = .5 * g.hy, sy = .5 * g.hx;
     for (int cell = blockIdx.x; cell < g.cells; cell += gridDim.x) {
         __syncthreads();
