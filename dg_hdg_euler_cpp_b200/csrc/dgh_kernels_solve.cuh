@@ -122,11 +122,13 @@ __device__ __forceinline__ void slab_fma(const uint4 &v, const float *y, unsigne
     acc = add2(acc, d);
 }
 
-// FP32 blocks at least this wide fetch of a diagonal square only the triangle of the sweep, L going forward and
-// U going back: fetched whole in both sweeps, the squares add a tenth to the bytes of 324-wide blocks.  65,536
+// FP32 blocks at least HALF_SQUARES wide fetch of a diagonal square only the triangle of the sweep, L going forward
+// and U going back: fetched whole in both sweeps, the squares add a tenth to the bytes of 324-wide blocks.  65,536
 // blocks of 324 (256, 144): 4.77 (2.71, 0.91) ms, with whole squares 5.06 (2.88, 0.98); 4,096 of 100: 55 against
-// 53 us, where the bytes do not bound it.  (FP16, bound by instructions: 3 to 6 % slower at 100 to 196.)
-constexpr int HALF_SQUARES = 128;
+// 53 us, where the bytes do not bound it.  (FP16, bound by instructions: 3 to 6 % slower at 100 to 196.)  Nor do
+// they with few warps at work, whose chains the choice of a square's lanes lengthens: 324 (256, 196, 144) wide, 576 blocks
+// 7 (10, 11, 17) % slower, 1,600 2 % faster (0, 0, 6 % slower), 2,500 4 (5, 6, 2) % faster.
+constexpr int HALF_SQUARES = 128, HALF_BLOCKS = 2368;
 
 __device__ __forceinline__ void ring_copy(unsigned dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -537,7 +539,7 @@ __device__ __forceinline__ void lu_solve_body(int bx, int G, const T *__restrict
                                               const int *__restrict__ perm, size_t stride, int m, int count,
                                               const double *__restrict__ rhs, double *__restrict__ z) {
     if (solve_whole<T>(m)) lu_solve_blocks<T, SlabWhole<T, false>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
-    else if (sizeof(T) == 4 && m >= HALF_SQUARES)
+    else if (sizeof(T) == 4 && m >= HALF_SQUARES && count >= HALF_BLOCKS)
         lu_solve_blocks<T, SlabStream<T, false, sizeof(T) == 4>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
     else lu_solve_blocks<T, SlabStream<T, false>>(bx, G, pool, aux, perm, stride, m, count, rhs, z);
 }
